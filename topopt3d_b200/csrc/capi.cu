@@ -232,7 +232,15 @@ int alloc_solver(Ctx &c) {
   }
   if (c.L > 2) A(c.gd_tmp, tpo::galerkin_dims_scratch(c.lev[1]));
   const int64_t nc = 3 * c.lev[c.L - 1].nn;
-  A(c.Adense, tpo::coarse_inverse_work(nc));   // inversion workspace
+  if (!c.inv.dev) {
+    tpo::coarse_inverse_plan(c.lev[c.L - 1].dims, c.inv);
+    A(c.inv.dev, c.inv.host.size());
+    CK(cudaMemcpyAsync(c.inv.dev, c.inv.host.data(), sizeof(int) * c.inv.host.size(),
+                       cudaMemcpyHostToDevice, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+    c.inv.host = std::vector<int>();
+  }
+  A(c.Adense, tpo::coarse_inverse_work(c.inv));   // inversion workspace
   A(c.Ainv, (size_t)(nc * nc));
   A(c.w64, 3 * c.nn);
 #undef A
@@ -252,7 +260,7 @@ void free_all(Ctx &c) {
   dfree(c.gk_G); c.gk_cap = 0; dfree(c.gd_tmp);
   dfree(c.l1_B); dfree(c.l1_rows); dfree(c.l1_C); c.l1_cap = 0; dfree(c.l1_cval);
   dfree(c.l1_cflag); dfree(c.l1_count); dfree(c.l1_fault); c.l1_bimg_ready = false;
-  dfree(c.Ainv); dfree(c.Adense); dfree(c.dev_info);
+  dfree(c.Ainv); dfree(c.Adense); dfree(c.inv.dev); dfree(c.dev_info);
   dfree(c.finv); dfree(c.taps_d);
   dfree(c.w64);
   dfree(c.Es64); dfree(c.dEsdz64); dfree(c.bk_buf); c.bk_n = 0; dfree(c.fq_buf); c.fq_n = 0; dfree(c.mma_buf); c.mma_n = 0;

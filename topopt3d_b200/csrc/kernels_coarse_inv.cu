@@ -1,5 +1,5 @@
-// Dense inverse of the coarsest-level operator, in place, by blocked
-// symmetric sweeps (Gauss-Jordan elimination without pivoting).
+// Dense inverse of the coarsest-level operator by blocked symmetric sweeps
+// (Gauss-Jordan elimination without pivoting) in a cyclic-reduction order.
 //
 // The coarsest operator is symmetric positive definite (the Galerkin
 // product of the clamped fine operator; the reference factorises it with a
@@ -7,28 +7,49 @@
 // complement -- is SPD and no pivoting is needed.  The V-cycle applies the
 // explicit inverse as one bandwidth-parallel matrix-vector product.
 //
-// The sweep of block K (P = A_KK^-1, F = the column block A_{.K}, G = F P):
+// The sweep of a pivot block K (P = A_KK^-1, F = the column block A_{.K},
+// G = F P):
 //   A_KK <- -P;  A_iK <- G_i;  A_Kj <- G_j^T;  A_ij <- A_ij - G_i F_j^T
-// keeps the matrix symmetric, so only the tiles on or below the diagonal
-// are updated (the row block K left of the diagonal holds G^T); after every
-// block has been swept the matrix is -A^-1, and a last pass negates it and
-// fills the upper triangle.  A sweep is two launches: F and G for every row
-// block (k_sw_fg), and the rank-64 update of the lower tiles on 64 x 64
-// tiles with FP64 tensor-core MMAs (k_sw_update), one CTA of which then
-// inverts the next
-// diagonal block by scalar Gauss-Jordan with a 4 x 4 block of it in each
-// thread's registers (sweep_diag; k_sw_diag for the first block).
+// keeps the matrix symmetric; after every block has been swept it is -A^-1.
+//
+// Order.  What bounds the inversion is the chain of pivot blocks (a few
+// microseconds of dependent arithmetic each), not its n^3 operations.  The
+// operator is a 27-point stencil, so with the unknowns grouped by the planes
+// normal to the longest dimension it is block tridiagonal, and every other
+// plane can be swept at the same time: pivot blocks that are not coupled
+// have a block-diagonal pivot matrix.  What is left is again a chain, of
+// half the length.  A 13 x 7 x 7 level (1,911 unknowns) takes 4 rounds of 3
+// blocks of 49, 12 dependent steps, where the natural order takes 30 steps
+// of 64; tiles that no pivot of a step couples are skipped (the structure is
+// worked out once per context on the host, plan_build).
+//
+// A step is two launches over task lists: F and G of every coupled (row
+// block, pivot) pair (k_ci_fg), and the updates of the lower tiles by
+// FP64 tensor-core MMAs (k_ci_update), where the tiles that are the next
+// step's pivots come first and are inverted in registers as soon as they
+// are updated (invert_tile), so the inversions overlap the other updates.
+// The matrix is kept as T x T tiles in plane order (T = 24 .. 64, the block
+// size rounded up, padded with the identity), each contiguous: every operand
+// is one run of 16-byte copies.
+//
+// Measured at 1,911 unknowns (serialised kernel time of one inversion): the
+// natural order in 64-blocks took 1,480 us, 36 us a step for the update
+// with the scalar inversion of the next block (22 us of it) and 12 us for F
+// and G; this form takes 356 us (12 x (6.4 + 19.7), fill 5, first pivots 13,
+// final pass 25), and FEAssemble of a 48 x 24 x 24 mesh 1.08 ms in place of
+// 2.18 ms.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
 #include "tpo_internal.h"
 
 namespace tpo {
 
 namespace {
 
-constexpr int kGB = 64;    // block size (rows / columns of a pivot block)
-constexpr int kGT = 256;   // threads per CTA: 16 x 16, 4 x 4 outputs each
-#ifndef TPO_SW_MINB
-#define TPO_SW_MINB 3
-#endif
+constexpr int kMaxTile = 64;
 
 // D (8 x 8) += A (8 x 4) B (4 x 8) in FP64 on the tensor cores.  Fragments
 // (PTX ISA, mma.m8n8k4 .f64): lane = 4 g + q holds A[g][q], B[q][g] and
@@ -39,302 +60,487 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// 8-byte asynchronous copy global -> shared; src_bytes 0 fills zeros (the
-// source address must still be valid)
-__device__ __forceinline__ void cp_async8(double *dst, const double *src, int src_bytes) {
+__device__ __forceinline__ void cp_async16(double *dst, const double *src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
-               "r"(src_bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// tile_gemm's operands in dynamic shared memory, the whole depth at once:
-// Xs[k][i] and, by layout, Ys[k][j] (YT) or Ys[j][k]; rows padded to 68
-// doubles so a warp's fragment reads fall on distinct bank pairs
-constexpr int kLd = kGB + 4;
-constexpr size_t kGemmSmem = 2 * sizeof(double) * kGB * kLd;
+__host__ __device__ constexpr int64_t tile_index(int I, int J) {   // I >= J
+  return (int64_t)I * (I + 1) / 2 + J;
+}
 
-// C (M x N, column-major, ldc) = (ACC ? C : 0) + s X Y for M, N <= 64 and a
-// depth Kd <= kGB, with X[i][k] = X[k * ldx + i] and Y[k][j] = Y[k * ldy + j]
-// (YT) or Y[j * ldy + k].  The operands are staged with asynchronous copies
-// and, with ACC, the thread's part of C is read while they are in flight;
-// every read of X and Y happens before the first write of C.  8 warps, each
-// a 16 x 32 block of the 64 x 64 tile as 2 x 4 tensor-core tiles of 8 x 8.
-template <bool ACC, bool YT>
-__device__ __forceinline__ void tile_gemm(double *smem, int M, int N, int Kd,
-                                          const double *X, int ldx, const double *Y,
-                                          int ldy, double *C, int ldc, double s) {
-  double *Xs = smem, *Ys = smem + kGB * kLd;
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int g = lane >> 2, q = lane & 3;
-  const int r0 = (w >> 1) * 16, c0 = (w & 1) * 32;
-  __syncthreads();   // the buffers are free (a previous use has finished)
-#pragma unroll 4
-  for (int e8 = 0; e8 < kGB * kGB / kGT; ++e8) {
-    const int e = t + e8 * kGT;
-    {
-      const int i = e % kGB, k = e / kGB;
-      const bool ok = i < M && k < Kd;
-      cp_async8(Xs + k * kLd + i, ok ? X + (int64_t)k * ldx + i : X, ok ? 8 : 0);
-    }
-    if (YT) {
-      const int j = e % kGB, k = e / kGB;
-      const bool ok = j < N && k < Kd;
-      cp_async8(Ys + k * kLd + j, ok ? Y + (int64_t)k * ldy + j : Y, ok ? 8 : 0);
-    } else {
-      const int k = e % kGB, j = e / kGB;
-      const bool ok = j < N && k < Kd;
-      cp_async8(Ys + j * kLd + k, ok ? Y + (int64_t)j * ldy + k : Y, ok ? 8 : 0);
-    }
+// rows of T doubles are staged at a stride of T + 4: T is a multiple of 8,
+// so four consecutive rows start 8 banks apart and the fragment reads (8
+// consecutive doubles of 4 rows) are free of conflicts
+template <int T>
+struct Tile {
+  static constexpr int kLd = T + 4;
+  static constexpr int kWarps = T / 8;        // one 8-row strip per warp
+  static constexpr int kThreads = 32 * kWarps;
+  static constexpr int kElems = T * T;
+  static constexpr size_t kSmem = 2 * sizeof(double) * T * kLd;
+};
+
+template <int T>
+__device__ __forceinline__ void stage_tile(double *dst, const double *src) {
+  for (int e = threadIdx.x; e < T * T / 2; e += Tile<T>::kThreads) {
+    const int r = e / (T / 2), c = 2 * (e % (T / 2));
+    cp_async16(dst + r * Tile<T>::kLd + c, src + r * T + c);
   }
-  double cv[2][4][2];
-  if (ACC) {
+}
+
+// the D-fragment pair (d[g][2q], d[g][2q+1]) of an 8 x 8 block as the two
+// A fragments (d[g][q], d[g][4 + q])
+__device__ __forceinline__ void d_to_a(double d0, double d1, int lane, double &a0, double &a1) {
+  const int q = lane & 3, s = (lane & ~3) + (q >> 1);
+  const double x0 = __shfl_sync(0xffffffffu, d0, s), x1 = __shfl_sync(0xffffffffu, d1, s);
+  const double y0 = __shfl_sync(0xffffffffu, d0, s + 2), y1 = __shfl_sync(0xffffffffu, d1, s + 2);
+  a0 = (q & 1) ? x1 : x0;
+  a1 = (q & 1) ? y1 : y0;
+}
+
+// -M^-1 of the symmetric T x T tile whose 8-row strip w each warp holds in
+// acc (D fragments of T / 8 blocks), by sweeps of 8 x 8 pivots: the block
+// column of the pivot goes to shared memory, every warp inverts the pivot
+// block for itself (scalar Gauss-Jordan by shuffles; one barrier per pivot)
+// and updates its strip with tensor-core MMAs.  A pivot that is not
+// positive records its dof + 1 in *info (the first one wins).
+// Fs: 2 x T x 12 doubles.
+template <int T>
+__device__ __forceinline__ void invert_tile(double (&acc)[T / 8][2], double *Fs, const int *dof,
+                                            int *info) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+  for (int kb = 0; kb < T / 8; ++kb) {
+    double *F = Fs + (kb & 1) * T * 12;
+    *reinterpret_cast<double2 *>(F + (8 * w + g) * 12 + 2 * q) =
+        make_double2(acc[kb][0], acc[kb][1]);
+    __syncthreads();
+    const double2 m = *reinterpret_cast<const double2 *>(F + (8 * kb + g) * 12 + 2 * q);
+    double m0 = m.x, m1 = m.y;
 #pragma unroll
-      for (int b = 0; b < 4; ++b)
+    for (int k = 0; k < 8; ++k) {
+      const double ms = (k & 1) ? m1 : m0;
+      const double p = __shfl_sync(0xffffffffu, ms, 4 * k + (k >> 1));
+      const double rk0 = __shfl_sync(0xffffffffu, m0, 4 * k + q);
+      const double rk1 = __shfl_sync(0xffffffffu, m1, 4 * k + q);
+      const double ck = __shfl_sync(0xffffffffu, ms, 4 * g + (k >> 1));
+      const bool ok = p > 0.0 && p < INFINITY;
+      if (!ok && threadIdx.x == 0) atomicCAS(info, 0, dof[8 * kb + k] + 1);
+      const double ip = ok ? 1.0 / p : 0.0;
+      const double r0 = rk0 * ip, r1 = rk1 * ip;
+      m0 = g == k ? r0 : fma(-ck, r0, m0);
+      m1 = g == k ? r1 : fma(-ck, r1, m1);
+      if (2 * q == k) m0 = g == k ? ip : -ck * ip;
+      if (2 * q + 1 == k) m1 = g == k ? ip : -ck * ip;
+    }
+    // P8 = (m0, m1); it is symmetric, so its A fragments are its B
+    // fragments too
+    double p0, p1;
+    d_to_a(m0, m1, lane, p0, p1);
+    double gd[2] = {0.0, 0.0}, a0, a1;
+    dmma(gd, F[(8 * w + g) * 12 + q], p0);
+    dmma(gd, F[(8 * w + g) * 12 + 4 + q], p1);
+    d_to_a(-gd[0], -gd[1], lane, a0, a1);
+    const bool own = w == kb;   // the pivot's strip becomes P8 F_j^T
+    if (own) {
+      a0 = p0;
+      a1 = p1;
+    }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int i = r0 + a * 8 + g, j = c0 + b * 8 + 2 * q + h;
-          cv[a][b][h] = (i < M && j < N) ? C[(int64_t)j * ldc + i] : 0.0;
-        }
+    for (int j = 0; j < T / 8; ++j) {
+      if (j == kb) continue;
+      if (own) acc[j][0] = acc[j][1] = 0.0;
+      dmma(acc[j], a0, F[(8 * j + g) * 12 + q]);
+      dmma(acc[j], a1, F[(8 * j + g) * 12 + 4 + q]);
+    }
+    acc[kb][0] = own ? -m0 : gd[0];
+    acc[kb][1] = own ? -m1 : gd[1];
   }
-  double acc[2][4][2];
+}
+
+// element (8w + g, 8j + 2q + h) of a column-major tile
+template <int T>
+__device__ __forceinline__ void load_strip(double (&acc)[T / 8][2], const double *tile) {
+  const int lane = threadIdx.x & 31, r = 8 * (threadIdx.x >> 5) + (lane >> 2), q = lane & 3;
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int j = 0; j < T / 8; ++j)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int h = 0; h < 2; ++h) acc[j][h] = tile[(8 * j + 2 * q + h) * T + r];
+}
+template <int T>
+__device__ __forceinline__ void store_strip(const double (&acc)[T / 8][2], double *tile,
+                                            double s) {
+  const int lane = threadIdx.x & 31, r = 8 * (threadIdx.x >> 5) + (lane >> 2), q = lane & 3;
+#pragma unroll
+  for (int j = 0; j < T / 8; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) tile[(8 * j + 2 * q + h) * T + r] = s * acc[j][h];
+}
+
+// inverts the pivot tile held in acc: P to the workspace, -P to the matrix
+template <int T>
+__device__ __forceinline__ void pivot_out(double (&acc)[T / 8][2], double *smem, int I,
+                                          double *W, double *P, const int *dofs, int *info) {
+  __syncthreads();   // the shared buffers are free
+  invert_tile<T>(acc, smem, dofs + I * T, info);
+  store_strip<T>(acc, W + tile_index(I, I) * T * T, 1.0);
+  store_strip<T>(acc, P, -1.0);
+}
+
+// the first step's pivots
+template <int T>
+__global__ void __launch_bounds__(Tile<T>::kThreads)
+    k_ci_pivots(const int *__restrict__ piv, double *W, double *P, const int *__restrict__ dofs,
+                int *info) {
+  extern __shared__ __align__(16) double smem[];
+  const int I = piv[blockIdx.x];
+  double acc[T / 8][2];
+  load_strip<T>(acc, W + tile_index(I, I) * T * T);
+  pivot_out<T>(acc, smem, I, W, P + (size_t)blockIdx.x * T * T, dofs, info);
+}
+
+// task (I, K, pivot slot): F_I = A_IK (the transposed tile (K, I) above the
+// diagonal) and G_I = F_I P; both to the workspace, [k][i], and G_I to the
+// matrix
+template <int T>
+__global__ void __launch_bounds__(Tile<T>::kThreads)
+    k_ci_fg(const int4 *__restrict__ tasks, double *W, const double *__restrict__ P, double *F,
+            double *G) {
+  extern __shared__ __align__(16) double smem[];
+  constexpr int ld = Tile<T>::kLd;
+  double *Xs = smem, *Ps = smem + T * ld;
+  const int4 t = tasks[blockIdx.x];
+  const int I = t.x, K = t.y;
+  const bool below = I > K;
+  double *a = W + (below ? tile_index(I, K) : tile_index(K, I)) * T * T;
+  stage_tile<T>(Xs, a);
+  stage_tile<T>(Ps, P + (size_t)t.z * T * T);
   cp_async_wait_all();
   __syncthreads();
-#pragma unroll 4
-  for (int k0 = 0; k0 < kGB; k0 += 4) {
-    double av[2], bv[4];
+  const int lane = threadIdx.x & 31, r0 = 8 * (threadIdx.x >> 5), g = lane >> 2, q = lane & 3;
+  double acc[T / 8][2];
 #pragma unroll
-    for (int a = 0; a < 2; ++a) av[a] = Xs[(k0 + q) * kLd + r0 + a * 8 + g];
+  for (int j = 0; j < T / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+#pragma unroll 2
+  for (int k0 = 0; k0 < T; k0 += 4) {
+    const double av = below ? Xs[(k0 + q) * ld + r0 + g] : Xs[(r0 + g) * ld + k0 + q];
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
-      bv[b] = YT ? Ys[(k0 + q) * kLd + c0 + b * 8 + g] : Ys[(c0 + b * 8 + g) * kLd + k0 + q];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) dmma(acc[a][b], av[a], bv[b]);
+    for (int j = 0; j < T / 8; ++j) dmma(acc[j], av, Ps[(k0 + q) * ld + 8 * j + g]);
   }
-  __syncthreads();   // C may alias an operand
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int i = r0 + a * 8 + g;
-    if (i >= M) continue;
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = c0 + b * 8 + 2 * q + h;
-        if (j >= N) continue;
-        C[(int64_t)j * ldc + i] = ACC ? fma(s, acc[a][b][h], cv[a][b][h]) : s * acc[a][b][h];
-      }
+  double *f = F + (size_t)blockIdx.x * T * T, *gw = G + (size_t)blockIdx.x * T * T;
+  for (int e = threadIdx.x; e < T * T; e += Tile<T>::kThreads) {
+    const int k = e / T, i = e % T;
+    f[e] = below ? Xs[k * ld + i] : Xs[i * ld + k];
   }
-}
-
-// P = A_KK^-1 of the bs x bs diagonal block at (K0, K0) by scalar
-// Gauss-Jordan; thread (tx, ty) keeps rows 4tx.. and columns 4ty.. in
-// registers, and each step broadcasts the pivot row and column through
-// shared memory (double-buffered, one barrier per step).  P goes to the
-// workspace (ld kGB) and -P to A.  A pivot that is not positive records
-// its global index + 1 in *info (the first one wins).
-__device__ __forceinline__ void sweep_diag(int n, double *A, int K0, int bs, double *P,
-                                           int *info) {
-  __shared__ double rowk[2][kGB], colk[2][kGB];
-  const int t = threadIdx.x, tx = t % 16, ty = t / 16;
-  const int r0 = tx * 4, c0 = ty * 4;
-  double m[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = r0 + a, cc = c0 + b;
-      // identity outside the block, so the padding never pivots on zero
-      m[a][b] = (r < bs && cc < bs) ? A[(int64_t)(K0 + cc) * n + K0 + r]
-                                    : (r == cc ? 1.0 : 0.0);
-    }
-#pragma unroll 4
-  for (int k = 0; k < kGB; ++k) {
-    const int buf = k & 1;
-    // publish the pivot row (owners: rows 4tx..4tx+3 hold k) and column
-    // (the row/column index is selected with unrolled compares so m stays
-    // in registers)
-    if ((k >> 2) == tx) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-        if (a == (k & 3)) {
-#pragma unroll
-          for (int b = 0; b < 4; ++b) rowk[buf][c0 + b] = m[a][b];
-        }
-    }
-    if ((k >> 2) == ty) {
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (b == (k & 3)) {
-#pragma unroll
-          for (int a = 0; a < 4; ++a) colk[buf][r0 + a] = m[a][b];
-        }
-    }
-    __syncthreads();
-    const double p = rowk[buf][k];
-    const bool ok = p > 0.0 && p < INFINITY;
-    if (!ok && t == 0 && k < bs) atomicCAS(info, 0, K0 + k + 1);
-    const double ip = ok ? 1.0 / p : 0.0;
-    double rk[4], ck[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) rk[b] = rowk[buf][c0 + b] * ip;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) ck[a] = colk[buf][r0 + a];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int r = r0 + a, cc = c0 + b;
-        double v = fma(-ck[a], rk[b], m[a][b]);   // generic entry
-        if (r == k) v = rk[b];                     // pivot row: a / p
-        if (cc == k) v = (r == k) ? ip : -ck[a] * ip;   // pivot column
-        m[a][b] = v;
-      }
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = r0 + a, cc = c0 + b;
-      if (r < bs && cc < bs) {
-        P[cc * kGB + r] = m[a][b];
-        A[(int64_t)(K0 + cc) * n + K0 + r] = -m[a][b];
-      }
-    }
-}
-
-__global__ void __launch_bounds__(kGT) k_sw_diag(int n, double *A, int K0, int bs,
-                                                  double *P, int *info) {
-  sweep_diag(n, A, K0, bs, P, info);
-}
-
-// CTA I (I != K): F_I = the rows of tile I of the column block K (below the
-// diagonal: tile (I, K); above: the transposed tile (K, I) of the row
-// block), and G_I = F_I P; both n x bs, column-major
-__global__ void __launch_bounds__(kGT, 3) k_sw_fg(int n, const double *A, int K0, int bs,
-                                               const double *P, double *F, double *G) {
-  const int I = blockIdx.x, i0 = I * kGB;
-  if (i0 == K0) return;
-  const int rows = min(kGB, n - i0);
-  // 16 independent copies per thread, unrolled so the loads overlap
-  if (i0 > K0) {
-#pragma unroll
-    for (int q = 0; q < kGB * kGB / kGT; ++q) {
-      const int e = threadIdx.x + q * kGT, i = e % kGB, k = e / kGB;
-      if (i < rows && k < bs) F[(int64_t)k * n + i0 + i] = A[(int64_t)(K0 + k) * n + i0 + i];
-    }
+  store_strip<T>(acc, gw, 1.0);
+  if (below) {
+    store_strip<T>(acc, a, 1.0);
   } else {
-    // A(K0 + k, i0 + i): k fastest for coalesced reads
 #pragma unroll
-    for (int q = 0; q < kGB * kGB / kGT; ++q) {
-      const int e = threadIdx.x + q * kGT, k = e % kGB, i = e / kGB;
-      if (i < rows && k < bs) F[(int64_t)k * n + i0 + i] = A[(int64_t)(i0 + i) * n + K0 + k];
-    }
-  }
-  __syncthreads();
-  extern __shared__ __align__(16) double gemm_smem[];
-  // G_I (rows x bs) = F_I (rows x bs) P (bs x bs); P[k][j] = P[j * kGB + k]
-  tile_gemm<false, false>(gemm_smem, rows, bs, bs, F + i0, n, P, kGB, G + i0, n, 1.0);
-}
-
-// lower tile (I, J), I >= J: the column block gets G_I, the row block left
-// of the diagonal G_J^T, every other tile A_IJ - G_I F_J^T.  The CTA of the
-// next diagonal tile (K+1, K+1) runs as block (0, 0), the first one
-// dispatched, and after its update inverts that block for the next sweep
-// (P and -P as k_sw_diag), so the diagonal inversion overlaps the rest of
-// the update instead of running alone between sweeps.
-__global__ void __launch_bounds__(kGT, TPO_SW_MINB) k_sw_update(int n, double *A, int K0, int bs,
-                                                    const double *F, const double *G,
-                                                    double *P, int *info) {
-  int I = blockIdx.x, J = blockIdx.y;
-  const int Kn = K0 / kGB + 1;   // the next diagonal tile
-  const bool look = Kn * kGB < n;
-  if (look) {
-    if (I == 0 && J == 0) I = J = Kn;
-    else if (I == Kn && J == Kn) I = J = 0;
-  }
-  if (J > I) return;
-  const int i0 = I * kGB, j0 = J * kGB;
-  const int M = min(kGB, n - i0), N = min(kGB, n - j0);
-  if (i0 == K0 && j0 == K0) return;   // the diagonal block: swept already
-  if (j0 == K0) {                      // A(i0 + i, K0 + k) = G(i0 + i, k)
-    for (int e = threadIdx.x; e < M * bs; e += kGT) {
-      const int i = e % M, k = e / M;
-      A[(int64_t)(K0 + k) * n + i0 + i] = G[(int64_t)k * n + i0 + i];
-    }
-    return;
-  }
-  if (i0 == K0) {                      // A(K0 + k, j0 + j) = G(j0 + j, k)
-    for (int e = threadIdx.x; e < N * bs; e += kGT) {
-      const int k = e % bs, j = e / bs;
-      A[(int64_t)(j0 + j) * n + K0 + k] = G[(int64_t)k * n + j0 + j];
-    }
-    return;
-  }
-  extern __shared__ __align__(16) double gemm_smem[];
-  // Y[k][j] = F(j0 + j, k) = F[k * n + j0 + j]
-  tile_gemm<true, true>(gemm_smem, M, N, bs, G + i0, n, F + j0, n, A + (int64_t)j0 * n + i0,
-                        n, -1.0);
-  if (look && I == Kn && J == Kn) {
-    __syncthreads();   // the tile's update is visible to the whole CTA
-    sweep_diag(n, A, i0, M, P, info);
+    for (int j = 0; j < T / 8; ++j)   // element (k = 8j + 2q + h, i) of tile (K, I)
+      *reinterpret_cast<double2 *>(a + (r0 + g) * T + 8 * j + 2 * q) =
+          make_double2(acc[j][0], acc[j][1]);
   }
 }
 
-// A <- -A on the lower triangle, mirrored into the upper one
-__global__ void k_sw_final(int n, double *A) {
+// task (tile I | J << 16, first pair, pairs, pivot slot of the next step or
+// -1): A_IJ -= sum over the pairs (G index, F index) of G_I F_J^T
+template <int T>
+__global__ void __launch_bounds__(Tile<T>::kThreads)
+    k_ci_update(const int4 *__restrict__ tasks, const int2 *__restrict__ pairs, double *W,
+                const double *__restrict__ F, const double *__restrict__ G, double *P,
+                const int *__restrict__ dofs, int *info) {
+  extern __shared__ __align__(16) double smem[];
+  constexpr int ld = Tile<T>::kLd;
+  double *Gs = smem, *Fs = smem + T * ld;
+  const int4 t = tasks[blockIdx.x];
+  const int I = t.x & 0xffff, J = t.x >> 16;
+  double *a = W + tile_index(I, J) * T * T;
+  const int lane = threadIdx.x & 31, r0 = 8 * (threadIdx.x >> 5), g = lane >> 2, q = lane & 3;
+  double acc[T / 8][2];
+  for (int p = 0; p < t.z; ++p) {
+    const int2 pr = pairs[t.y + p];
+    if (p) __syncthreads();
+    stage_tile<T>(Gs, G + (size_t)pr.x * T * T);
+    stage_tile<T>(Fs, F + (size_t)pr.y * T * T);
+    if (p == 0) load_strip<T>(acc, a);   // while the copies are in flight
+    cp_async_wait_all();
+    __syncthreads();
+#pragma unroll 2
+    for (int k0 = 0; k0 < T; k0 += 4) {
+      const double av = -Gs[(k0 + q) * ld + r0 + g];
+#pragma unroll
+      for (int j = 0; j < T / 8; ++j) dmma(acc[j], av, Fs[(k0 + q) * ld + 8 * j + g]);
+    }
+  }
+  if (t.z == 0) load_strip<T>(acc, a);
+  if (t.w >= 0)
+    pivot_out<T>(acc, smem, I, W, P + (size_t)t.w * T * T, dofs, info);
+  else
+    store_strip<T>(acc, a, 1.0);
+}
+
+// the stencil's entries on or below the diagonal to their tiles (zeroed
+// before), the identity on the padding
+__global__ void k_ci_fill(int nx, int ny, int nz, const double *__restrict__ S,
+                          const int *__restrict__ pos, const int *__restrict__ dofs, int nb,
+                          int T, double *__restrict__ W) {
+  const int64_t nn = (int64_t)nx * ny * nz, total = nn * 243;
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t st = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t t = t0; t < total; t += st) {
+    const int q = (int)(t / nn);
+    const int64_t n = t - (int64_t)q * nn;
+    const int b = q / 9, r = (q % 9) / 3, s = q % 3;
+    const int mi = (int)(n % nx) + b % 3 - 1, mj = (int)((n / nx) % ny) + (b / 3) % 3 - 1,
+              mk = (int)(n / ((int64_t)nx * ny)) + b / 9 - 1;
+    if (mi < 0 || mi >= nx || mj < 0 || mj >= ny || mk < 0 || mk >= nz) continue;
+    const int64_t m = ((int64_t)mk * ny + mj) * nx + mi;
+    const int pi = pos[3 * n + r], pj = pos[3 * m + s];
+    const int I = pi / T, J = pj / T;
+    if (I < J) continue;
+    W[tile_index(I, J) * T * T + (pj % T) * T + pi % T] = S[t];
+  }
+  for (int64_t t = t0; t < (int64_t)nb * T; t += st)
+    if (dofs[t] < 0) {
+      const int I = (int)(t / T), o = (int)(t % T);
+      W[tile_index(I, I) * T * T + o * T + o] = 1.0;
+    }
+}
+
+// Ainv (n x n, dof order) = -W, one CTA per tile on or below the diagonal
+__global__ void k_ci_final(int n, int T, const int *__restrict__ dofs,
+                           const double *__restrict__ W, double *__restrict__ Ainv) {
+  extern __shared__ __align__(16) double smem[];
   const int I = blockIdx.x, J = blockIdx.y;
   if (J > I) return;
-  const int i0 = I * kGB, j0 = J * kGB;
-  const int M = min(kGB, n - i0), N = min(kGB, n - j0);
-  for (int e = threadIdx.x; e < M * N; e += blockDim.x) {
-    const int i = e % M, j = e / M;
-    const int gi = i0 + i, gj = j0 + j;
-    if (gi < gj) continue;   // diagonal tiles: the lower half writes both
-    const double v = -A[(int64_t)gj * n + gi];
-    A[(int64_t)gj * n + gi] = v;
-    if (gi != gj) A[(int64_t)gi * n + gj] = v;
+  const double *a = W + tile_index(I, J) * T * T;
+  for (int e = threadIdx.x; e < T * T; e += blockDim.x)
+    smem[(e / T) * (T + 1) + e % T] = -a[e];   // [column][row]
+  __syncthreads();
+  for (int e = threadIdx.x; e < T * T; e += blockDim.x) {
+    const int u = e / T, v = e % T;
+    const int di = dofs[I * T + u], dj = dofs[J * T + v];
+    if (di >= 0 && dj >= 0) Ainv[(int64_t)di * n + dj] = smem[v * (T + 1) + u];
+    if (I != J) {
+      const int dr = dofs[J * T + u], dc = dofs[I * T + v];
+      if (dr >= 0 && dc >= 0) Ainv[(int64_t)dr * n + dc] = smem[u * (T + 1) + v];
+    }
+  }
+}
+
+template <int T>
+void run_steps(const CoarseInvPlan &pl, double *work, int *info, cudaStream_t s) {
+  double *W = work, *P = W + tile_index(pl.nb, 0) * T * T;
+  double *F = P + (size_t)pl.max_pivots * T * T, *G = F + (size_t)pl.max_fg * T * T;
+  const int4 *fg = reinterpret_cast<const int4 *>(pl.dev + pl.off_fg);
+  const int4 *up = reinterpret_cast<const int4 *>(pl.dev + pl.off_up);
+  const int2 *pairs = reinterpret_cast<const int2 *>(pl.dev + pl.off_pairs);
+  const int *dofs = pl.dev + pl.off_dofs;
+  const size_t sm = Tile<T>::kSmem;
+  static unsigned long long attr_set = 0;   // bit per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!((attr_set >> (dev & 63)) & 1ull)) {
+    cudaFuncSetAttribute(k_ci_pivots<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_ci_fg<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_ci_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    attr_set |= 1ull << (dev & 63);
+  }
+  constexpr int th = Tile<T>::kThreads;
+  count_launch();
+  k_ci_pivots<T><<<pl.first_pivots, th, sm, s>>>(pl.dev + pl.off_piv, W, P, dofs, info);
+  for (const CoarseInvPlan::Step &q : pl.steps) {
+    if (q.nfg) {
+      count_launch();
+      k_ci_fg<T><<<q.nfg, th, sm, s>>>(fg + q.fg, W, P, F, G);
+    }
+    if (q.nup) {
+      count_launch();
+      k_ci_update<T><<<q.nup, th, sm, s>>>(up + q.up, pairs, W, F, G, P, dofs, info);
+    }
   }
 }
 
 }  // namespace
 
-size_t coarse_inverse_work(int64_t n) { return 2 * (size_t)n * kGB + kGB * kGB; }
+// The blocks, the elimination order and the task lists of a level of d[0] x
+// d[1] x d[2] nodes (host arrays in pl.host; the caller uploads them).
+void coarse_inverse_plan(const int d[3], CoarseInvPlan &pl) {
+  const int D = (d[0] >= d[1] && d[0] >= d[2]) ? 0 : (d[1] >= d[2] ? 1 : 2);
+  const int planes = d[D];
+  const int m = 3 * (d[0] * d[1] * d[2] / planes);   // unknowns of one plane
+  // short planes are taken several at a time, long ones in several blocks
+  const int grp = std::max(1, std::min(planes, kMaxTile / m));
+  const int np = (planes + grp - 1) / grp, mp = grp * m;
+  const int bpp = (mp + kMaxTile - 1) / kMaxTile;     // blocks per plane group
+  const int bs = (mp + bpp - 1) / bpp;
+  // a level has at least 2 nodes per dimension, so m >= 12 and the blocks
+  // are of 24 (2 x 2 x 2 nodes) or 33 .. 64 unknowns
+  const int T = bs <= 24 ? 24 : std::max(40, (bs + 7) / 8 * 8);
+  const int nb = np * bpp;
+  pl.T = T;
+  pl.nb = nb;
+  pl.n = 3LL * d[0] * d[1] * d[2];
+  // position of each dof: plane group along D, then the nodes of its planes
+  // in the level's own order, in blocks of bs
+  std::vector<int> pos(pl.n), dofs((size_t)nb * T, -1);
+  std::vector<int> fill(np, 0);
+  for (int k = 0; k < d[2]; ++k)
+    for (int j = 0; j < d[1]; ++j)
+      for (int i = 0; i < d[0]; ++i) {
+        const int c[3] = {i, j, k};
+        const int g = c[D] / grp, n = (k * d[1] + j) * d[0] + i;
+        for (int r = 0; r < 3; ++r) {
+          const int o = fill[g]++;
+          const int p = (g * bpp + o / bs) * T + o % bs;
+          pos[3 * n + r] = p;
+          dofs[p] = 3 * n + r;
+        }
+      }
+  // coupled block pairs
+  std::vector<uint8_t> nz((size_t)nb * nb, 0);
+  for (int k = 0; k < d[2]; ++k)
+    for (int j = 0; j < d[1]; ++j)
+      for (int i = 0; i < d[0]; ++i)
+        for (int b = 0; b < 27; ++b) {
+          const int mi = i + b % 3 - 1, mj = j + (b / 3) % 3 - 1, mk = k + b / 9 - 1;
+          if (mi < 0 || mj < 0 || mk < 0 || mi >= d[0] || mj >= d[1] || mk >= d[2]) continue;
+          const int n = (k * d[1] + j) * d[0] + i, q = (mk * d[1] + mj) * d[0] + mi;
+          for (int r = 0; r < 3; ++r)
+            for (int s = 0; s < 3; ++s)
+              nz[(size_t)(pos[3 * n + r] / T) * nb + pos[3 * q + s] / T] = 1;
+        }
+  // rounds of alternate plane groups; block b of every group of a round is
+  // one step as long as the groups are uncoupled
+  std::vector<std::vector<int>> steps;
+  std::vector<int> chain(np);
+  for (int g = 0; g < np; ++g) chain[g] = g;
+  std::vector<uint8_t> st = nz;   // structure as the elimination proceeds
+  auto coupled = [&](int a, int b) { return st[(size_t)a * nb + b] != 0; };
+  std::vector<int> nzr;
+  auto eliminate = [&](int k) {
+    nzr.clear();
+    for (int i = 0; i < nb; ++i)
+      if (i != k && coupled(i, k)) nzr.push_back(i);
+    for (int a : nzr)
+      for (int b : nzr) st[(size_t)a * nb + b] = 1;
+  };
+  while (!chain.empty()) {
+    std::vector<int> round, rest;
+    for (size_t t = 0; t < chain.size(); ++t) (t % 2 ? rest : round).push_back(chain[t]);
+    for (int b = 0; b < bpp; ++b) {
+      std::vector<int> todo;
+      for (int g : round) todo.push_back(g * bpp + b);
+      while (!todo.empty()) {
+        std::vector<int> now, later;
+        for (int k : todo) {
+          bool free = true;
+          for (int o : now) free = free && !coupled(k, o);
+          (free ? now : later).push_back(k);
+        }
+        steps.push_back(now);
+        for (int k : now) eliminate(k);
+        todo.swap(later);
+      }
+    }
+    chain.swap(rest);
+  }
+  // task lists
+  std::vector<int> fg, up, pairs;
+  st = nz;
+  pl.max_pivots = 1;
+  pl.max_fg = 1;
+  pl.steps.clear();
+  for (size_t q = 0; q < steps.size(); ++q) {
+    const std::vector<int> &piv = steps[q];
+    pl.max_pivots = std::max(pl.max_pivots, (int)piv.size());
+    CoarseInvPlan::Step S{};
+    S.fg = (int)(fg.size() / 4);
+    S.up = (int)(up.size() / 4);
+    std::vector<uint8_t> is_piv(nb, 0);
+    for (int k : piv) is_piv[k] = 1;
+    // index of (I, pivot) among this step's F and G tiles, per row block
+    std::vector<std::vector<std::pair<int, int>>> of(nb);
+    int nfg = 0;
+    for (size_t p = 0; p < piv.size(); ++p)
+      for (int I = 0; I < nb; ++I)
+        if (I != piv[p] && coupled(I, piv[p])) {
+          of[I].push_back({(int)p, nfg++});
+          fg.insert(fg.end(), {I, piv[p], (int)p, 0});
+        }
+    S.nfg = nfg;
+    pl.max_fg = std::max(pl.max_fg, nfg);
+    std::vector<int> slot(nb, -1);
+    if (q + 1 < steps.size())
+      for (size_t p = 0; p < steps[q + 1].size(); ++p) slot[steps[q + 1][p]] = (int)p;
+    auto task = [&](int I, int J) {
+      const int next = I == J ? slot[I] : -1;
+      const int first = (int)(pairs.size() / 2);
+      int cnt = 0;
+      if (!is_piv[I] && !is_piv[J])
+        for (auto &a : of[I])
+          for (auto &b : of[J])
+            if (a.first == b.first) {
+              pairs.insert(pairs.end(), {a.second, b.second});
+              ++cnt;
+            }
+      if (cnt || next >= 0) up.insert(up.end(), {I | (J << 16), first, cnt, next});
+    };
+    for (int I = 0; I < nb; ++I)   // the next step's pivots first
+      if (slot[I] >= 0) task(I, I);
+    for (int I = 0; I < nb; ++I)
+      for (int J = 0; J <= I; ++J)
+        if (!(I == J && slot[I] >= 0)) task(I, J);
+    S.nup = (int)(up.size() / 4) - S.up;
+    pl.steps.push_back(S);
+    for (int k : piv) eliminate(k);
+  }
+  pl.first_pivots = (int)steps[0].size();
+  // one device array; the task lists (int4, int2) first, for their alignment
+  pl.host.clear();
+  auto put = [&](const std::vector<int> &v) {
+    const size_t o = pl.host.size();
+    pl.host.insert(pl.host.end(), v.begin(), v.end());
+    while (pl.host.size() % 4) pl.host.push_back(0);
+    return o;
+  };
+  pl.off_fg = put(fg);
+  pl.off_up = put(up);
+  pl.off_pairs = put(pairs);
+  pl.off_piv = put(steps[0]);
+  pl.off_dofs = put(dofs);
+  pl.off_pos = put(pos);
+}
 
-void launch_coarse_inverse(int64_t n64, double *A, double *work, int *info, cudaStream_t s) {
-  const int n = (int)n64;
-  const int nt = (n + kGB - 1) / kGB;
-  double *P = work, *F = work + kGB * kGB, *G = F + (size_t)n * kGB;
-  static unsigned long long attr_set = 0;   // bit per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!((attr_set >> (dev & 63)) & 1ull)) {
-    cudaFuncSetAttribute(k_sw_fg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
-    cudaFuncSetAttribute(k_sw_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kGemmSmem);
-    attr_set |= 1ull << (dev & 63);
-  }
+size_t coarse_inverse_work(const CoarseInvPlan &pl) {
+  const size_t tile = (size_t)pl.T * pl.T;
+  return tile * (tile_index(pl.nb, 0) + pl.max_pivots + 2 * (size_t)pl.max_fg);
+}
+
+void launch_coarse_inverse(const Level &v, const double *S, const CoarseInvPlan &pl,
+                           double *Ainv, double *work, int *info, cudaStream_t s) {
+  const int T = pl.T, nb = pl.nb;
   cudaMemsetAsync(info, 0, sizeof(int), s);
-  count_launch();
-  k_sw_diag<<<1, kGT, 0, s>>>(n, A, 0, std::min(kGB, n), P, info);
-  for (int K0 = 0; K0 < n; K0 += kGB) {
-    const int bs = std::min(kGB, n - K0);
-    count_launch(2);
-    k_sw_fg<<<nt, kGT, kGemmSmem, s>>>(n, A, K0, bs, P, F, G);
-    k_sw_update<<<dim3(nt, nt), kGT, kGemmSmem, s>>>(n, A, K0, bs, F, G, P, info);
+  cudaMemsetAsync(work, 0, sizeof(double) * tile_index(nb, 0) * T * T, s);
+  count_launch(2);
+  const int64_t g = std::min<int64_t>((v.nn * 243 + 255) / 256, 148 * 32);
+  k_ci_fill<<<(int)g, 256, 0, s>>>(v.dims[0], v.dims[1], v.dims[2], S, pl.dev + pl.off_pos,
+                                   pl.dev + pl.off_dofs, nb, T, work);
+  switch (T) {
+    case 24: run_steps<24>(pl, work, info, s); break;
+    case 40: run_steps<40>(pl, work, info, s); break;
+    case 48: run_steps<48>(pl, work, info, s); break;
+    case 56: run_steps<56>(pl, work, info, s); break;
+    default: run_steps<64>(pl, work, info, s); break;
   }
-  count_launch();
-  k_sw_final<<<dim3(nt, nt), kGT, 0, s>>>(n, A);
+  k_ci_final<<<dim3(nb, nb), 256, sizeof(double) * T * (T + 1), s>>>((int)pl.n, T,
+                                                                     pl.dev + pl.off_dofs, work,
+                                                                     Ainv);
 }
 
 }  // namespace tpo

@@ -538,23 +538,6 @@ __global__ void k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz,
   }
 }
 
-__global__ void k_to_dense(int nx, int ny, int nz, const double *__restrict__ S,
-                           double *__restrict__ A) {
-  const int64_t nn = (int64_t)nx * ny * nz, n3 = 3 * nn;
-  const int64_t total = nn * 27 * 9;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int q = (int)(t / nn);
-    const int64_t n = t - (int64_t)q * nn;
-    const int nb = q / 9, rs = q % 9, r = rs / 3, s = rs % 3;
-    const int i = n % nx, j = (n / nx) % ny, k = n / ((int64_t)nx * ny);
-    const int mi = i + nb % 3 - 1, mj = j + (nb / 3) % 3 - 1, mk = k + nb / 9 - 1;
-    if (mi < 0 || mi >= nx || mj < 0 || mj >= ny || mk < 0 || mk >= nz) continue;
-    const int64_t m = ((int64_t)mk * ny + mj) * nx + mi;
-    A[(3 * n + r) * n3 + 3 * m + s] = S[t];
-  }
-}
-
 // x = Ainv b, one warp per row, FP64 accumulation
 template <typename T>
 __global__ void k_coarse_gemv(int64_t n, const double *__restrict__ A,
@@ -799,15 +782,6 @@ template void launch_prolong_add<double>(const Level &, const Level &,
 template void launch_prolong_add<float>(const Level &, const Level &,
                                         const float *, float *, cudaStream_t,
                                         int);
-
-void launch_to_dense(const Level &v, const double *S, double *A,
-                     cudaStream_t s) {
-  count_launch();
-  const int64_t n3 = 3 * v.nn;
-  cudaMemsetAsync(A, 0, sizeof(double) * n3 * n3, s);
-  k_to_dense<<<grid_for(v.nn * 243, 256), 256, 0, s>>>(v.dims[0], v.dims[1],
-                                                       v.dims[2], S, A);
-}
 
 namespace {
 __global__ void k_soa_to_aos(int64_t nn, const double *__restrict__ S,

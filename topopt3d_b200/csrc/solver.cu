@@ -654,15 +654,14 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
     }
   }
   CK(cudaGetLastError());
-  // coarsest level: the explicit inverse of the dense operator (blocked
+  // coarsest level: the explicit inverse of its operator (blocked
   // Gauss-Jordan, kernels_coarse_inv.cu) for a bandwidth-parallel GEMV
   // inside the V-cycle
   Level &cl = c.lev[c.L - 1];
   const double *Sc = (c.L == 1) ? c.S0 : cl.S64;
   const int64_t nc = 3 * cl.nn;
   c.nc = nc;
-  launch_to_dense(cl, Sc, c.Ainv, s);
-  launch_coarse_inverse(nc, c.Ainv, c.Adense, c.dev_info, s);
+  launch_coarse_inverse(cl, Sc, c.inv, c.Ainv, c.Adense, c.dev_info, s);
   CK(cudaGetLastError());
   int info_h = 0, l1_fault_h = 0;
   unsigned int l1_rows_h = 0;

@@ -92,6 +92,22 @@ struct Level {
         *a32 = nullptr, *e32 = nullptr, *w32 = nullptr;
 };
 
+// The coarsest inverse's elimination plan (kernels_coarse_inv.cu): tile size,
+// blocks, unknowns, the steps' ranges in the task lists, and the lists
+// (offsets into one int array, host until uploaded, then dev)
+struct CoarseInvPlan {
+  struct Step {
+    int fg, nfg, up, nup;
+  };
+  int T = 0, nb = 0;
+  int64_t n = 0;
+  int first_pivots = 0, max_pivots = 0, max_fg = 0;
+  std::vector<Step> steps;
+  std::vector<int> host;
+  size_t off_fg = 0, off_up = 0, off_pairs = 0, off_piv = 0, off_dofs = 0, off_pos = 0;
+  int *dev = nullptr;
+};
+
 // side streams of the set-up (per-level power iterations)
 constexpr int kAuxStreams = 4;
 // GMG levels of one context
@@ -216,6 +232,7 @@ struct Ctx {
   size_t io_bytes = 0;
 
   // coarsest inverse
+  CoarseInvPlan inv;
   double *Adense = nullptr;     // workspace of the coarsest inversion
   int *dev_info = nullptr;
 
@@ -363,17 +380,17 @@ void launch_restrict(const Level &fine, const Level &coarse, const T *rf,
 template <typename T>
 void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc,
                         T *xf, cudaStream_t s, int nb = 1);
-void launch_to_dense(const Level &v, const double *S, double *A,
-                     cudaStream_t s);
 // stencil SoA S[(nb*9 + 3r+s)*nn + n] -> node-major A[n*243 + (3r+s)*27 + nb]
 // (FP64 and an FP32 copy)
 void launch_soa_to_aos(int64_t nn, const double *S, double *A64, float *A32,
                        cudaStream_t s);
-// A (n x n, column-major, SPD) <- A^-1 in place by blocked Gauss-Jordan
-// (kernels_coarse_inv.cu); work holds coarse_inverse_work(n) doubles; *info
-// becomes the global index + 1 of the first pivot that is not positive
-size_t coarse_inverse_work(int64_t n);
-void launch_coarse_inverse(int64_t n, double *A, double *work, int *info, cudaStream_t s);
+// Ainv (n x n) = the inverse of the level's SPD stencil operator S
+// (kernels_coarse_inv.cu); work holds coarse_inverse_work(plan) doubles;
+// *info becomes the index + 1 of the first dof whose pivot is not positive
+void coarse_inverse_plan(const int dims[3], CoarseInvPlan &plan);
+size_t coarse_inverse_work(const CoarseInvPlan &plan);
+void launch_coarse_inverse(const Level &v, const double *S, const CoarseInvPlan &plan,
+                           double *Ainv, double *work, int *info, cudaStream_t s);
 template <typename T>
 void launch_coarse_gemv(int64_t n, const double *Ainv, const T *b, T *x,
                         cudaStream_t s, int nb = 1);
