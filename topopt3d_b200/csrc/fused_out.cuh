@@ -1,6 +1,6 @@
 // Input and epilogue forms shared by the level-1 operator kernels (the
 // half-stored stencil, kernels_mg.cu; the tensor-core form, kernels_l1tc.cu).
-// They match the fine-level kernel's (kernels_apply_staged.cu, finish_dof):
+// They match the fine-level kernel's (kernels_apply_staged.cu):
 // IN_U reads u, IN_CHEB forms the Chebyshev start invtheta D^-1 b on the
 // fly; OUT_Y / OUT_RESID / OUT_CHEB2 / OUT_POST0 / OUT_POST1 write Au,
 // b - Au or the fused Chebyshev(2) updates.
@@ -18,9 +18,9 @@ __device__ __forceinline__ T sym_in(const ApplyArgs<T> &a, int i) {
 
 // the epilogue on values already loaded: bi = b[i], di = dinv[i],
 // y2i = y2[i] (each read only by the forms that use it)
-template <typename T, int OUT>
-__device__ __forceinline__ void sym_out_v(const ApplyArgs<T> &a, int i, T Au, T u, T bi,
-                                          T di, T y2i) {
+template <typename T, int OUT, typename I>
+__device__ __forceinline__ void sym_out_v(const ApplyArgs<T> &a, I i, T Au, T u, T bi, T di,
+                                          T y2i) {
   if (OUT == OUT_Y) {
     a.y[i] = Au;
   } else if (OUT == OUT_RESID) {

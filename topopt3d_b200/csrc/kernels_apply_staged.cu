@@ -36,6 +36,7 @@
 // one plane ahead.  The pipeline: at step p the plane p is loaded into
 // edges and faces, element layer p-1 is applied, the faces of plane p-1 are
 // complete, and nodes of plane p-2 are written.
+#include "fused_out.cuh"
 #include "modal.cuh"
 
 namespace tpo {
@@ -45,15 +46,8 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kLanesOut = 30;   // written nodes per tile row
 
-// the input vector of dof i: u_i (IN_U) or the Chebyshev start from a zero
-// guess, invtheta * dinv_i * b_i (IN_CHEB)
-template <typename T, int IN>
-__device__ __forceinline__ T input_value(const ApplyArgs<T> &a, int64_t i) {
-  if (IN == IN_CHEB) return a.invtheta * (__ldg(a.dinv + i) * __ldg(a.b + i));
-  return __ldg(a.u + i);
-}
-
-// epilogue of dof i with Au_i = (M K M u + (1-M) u)_i and u_i the input:
+// epilogue of dof i with Au_i = (M K M u + (1-M) u)_i and u_i the input; bi,
+// di, y2i are b_i, dinv_i, y2_i where the form needs them (OutNeeds):
 //   OUT_Y     y = Au
 //   OUT_RESID y = b - Au
 //   OUT_CHEB2 Chebyshev(2) from a zero guess, input d0 = invtheta dinv b:
@@ -62,26 +56,47 @@ __device__ __forceinline__ T input_value(const ApplyArgs<T> &a, int64_t i) {
 //             y = d0, y2 = u + d0
 //   OUT_POST1 second step, input d0 = u (so r0 = theta d0):
 //             d1 = c1 d0 + c2 (theta d0 - dinv Au); y = x1 + d1 (x1 = y2)
-template <typename T, int OUT>
-__device__ __forceinline__ void finish_dof(const ApplyArgs<T> &a, int64_t i,
-                                           T Au, T u) {
-  if (OUT == OUT_Y) {
-    a.y[i] = Au;
-  } else if (OUT == OUT_RESID) {
-    a.y[i] = __ldg(a.b + i) - Au;
-  } else if (OUT == OUT_CHEB2) {
-    const T di = __ldg(a.dinv + i), bi = __ldg(a.b + i);
-    const T r1 = di * bi - di * Au;
-    a.y[i] = u + (a.c1 * u + a.c2 * r1);
-  } else if (OUT == OUT_POST0) {
-    const T d0 = a.invtheta * (__ldg(a.dinv + i) * (__ldg(a.b + i) - Au));
-    a.y[i] = d0;
-    a.y2[i] = u + d0;
-  } else {   // OUT_POST1
-    const T r1 = a.theta * u - __ldg(a.dinv + i) * Au;
-    a.y[i] = a.y2[i] + (a.c1 * u + a.c2 * r1);
-  }
+// (sym_out_v, fused_out.cuh)
+
+// Operands that a thread reads for its own node only -- b, dinv, y2 of the
+// epilogue, and b and dinv of the IN_CHEB input -- are copied to shared
+// memory asynchronously one plane ahead.  A load at the point of use stalls
+// the 16 warps of an SM for its latency in every plane, and there are no
+// registers left to prefetch into.  At 192x96x96, before and after (us, FP32
+// / FP64; the plain product takes 33 / 61): OUT_CHEB2 58 -> 40 / 130 -> 77,
+// OUT_POST0 51 -> 41 / 109 -> 81, OUT_POST1 53 -> 40 / 121 -> 74, OUT_RESID
+// 38 / 94 -> 70; 8 columns of 128x64x64 in FP32: 152 -> 104, 135 -> 107,
+// 146 -> 104 and 123 -> 99.
+__device__ __forceinline__ void copy_async(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
 }
+__device__ __forceinline__ void copy_async(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+// staged arrays and planes: IN_CHEB keeps b and dinv of 4 planes (loaded
+// ahead, input, and two planes later the epilogue) and the row above the
+// tile; the other forms 2 planes of what their epilogue reads; the
+// Chebyshev forms with IN_U also keep their input of 3 planes (4 slots)
+template <int IN, int OUT>
+struct Staged {
+  static constexpr bool kIn = IN == IN_CHEB;
+  static constexpr bool kB = OutNeeds<OUT>::b, kD = OutNeeds<OUT>::dinv, kY = OutNeeds<OUT>::y2;
+  static constexpr bool kU = !kIn && (OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1);
+  static constexpr int kArrays = kIn ? 2 : int(kB) + int(kD) + int(kY);
+  static constexpr int kSlots = kIn ? 4 : 2;
+  static constexpr int kSlotB = 0, kSlotD = kIn ? 1 : int(kB), kSlotY = int(kB) + int(kD);
+  static constexpr int planes() { return kArrays * kSlots + (kU ? 4 : 0); }
+};
 
 // six values per thread in shared memory with 16-byte accesses: FP32 as one
 // float4 (v0, w0, v1, w1) and one float2 (v2, w2) per lane; FP64 as three
@@ -144,7 +159,6 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     k_apply_staged(int nelx, int nely, int nelz, int zchunk,
                    const T *__restrict__ E, const uint8_t *__restrict__ fix,
                    const ApplyArgs<T> args_in, const Kh<T> kh) {
-  constexpr bool kNeedU = OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1;
   const int Nx = nelx + 1, Ny = nely + 1, Nz = nelz + 1;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int gx = (int)blockIdx.x * kLanesOut - 1 + tx;
@@ -188,33 +202,76 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
   se.bind(smem_raw, 2 * kRows);
   sc.bind(smem_raw + 2 * kRows * Six<T>::bytes_per_row(), 2 * kRows);
 
+  // the staged operands, 3 values per thread: element (array, slot, row,
+  // lane, component)
+  using Sg = Staged<IN, OUT>;
+  T *stage = reinterpret_cast<T *>(smem_raw + 4 * kRows * Six<T>::bytes_per_row());
+  auto slot_at = [&](int arr, int z, int row) -> T * {
+    return stage + ((arr * Sg::kSlots + (z & (Sg::kSlots - 1))) * kRows + row) * 96 + 3 * tx;
+  };
+  T *const ring_u = stage + Sg::kArrays * Sg::kSlots * kRows * 96;
+  auto ring_at = [&](int z) -> T * { return ring_u + ((z & 3) * kRows + ty) * 96 + 3 * tx; };
+
   // prefetched next plane: own node, the row-above node (last row), the
-  // fixed-component bits and the modulus of the element layer below it
+  // fixed-component bits (all set where there is no node, so its value is
+  // masked) and the modulus of the element layer below it
   T pu[3] = {T(0), T(0), T(0)}, pq[3] = {T(0), T(0), T(0)};
-  unsigned pf = 0u, pf2 = 0u;
+  unsigned pf = 7u, pf2 = 7u;
   T pE = T(0);
   auto fetch = [&](int z) {   // z is uniform over the CTA
     // fresh zeros every plane let the loads target renamed registers
-    pf = pf2 = 0u;
+    pf = pf2 = 7u;
+    if (!Sg::kIn) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) pu[c] = pq[c] = T(0);
+      for (int c = 0; c < 3; ++c) pu[c] = pq[c] = T(0);
+    }
     pE = T(0);
     if (z >= 0 && z < Nz) {
       const int n = nofs + z * NP;
       if (nin) {
         pf = __ldg(fix + n);
+        if (Sg::kIn) {
+          T *db = slot_at(Sg::kSlotB, z, ty), *dd = slot_at(Sg::kSlotD, z, ty);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) pu[c] = input_value<T, IN>(args, 3 * (int64_t)n + c);
+          for (int c = 0; c < 3; ++c) {
+            copy_async(db + c, args.b + 3 * (int64_t)n + c);
+            copy_async(dd + c, args.dinv + 3 * (int64_t)n + c);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) pu[c] = __ldg(args.u + 3 * (int64_t)n + c);
+        }
       }
       if (nin2) {
         const int n2 = nofs2 + z * NP;
         pf2 = __ldg(fix + n2);
+        if (Sg::kIn) {
+          T *db = slot_at(Sg::kSlotB, z, TY), *dd = slot_at(Sg::kSlotD, z, TY);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) pq[c] = input_value<T, IN>(args, 3 * (int64_t)n2 + c);
+          for (int c = 0; c < 3; ++c) {
+            copy_async(db + c, args.b + 3 * (int64_t)n2 + c);
+            copy_async(dd + c, args.dinv + 3 * (int64_t)n2 + c);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) pq[c] = __ldg(args.u + 3 * (int64_t)n2 + c);
+        }
       }
     }
     const int ez = z - 1;
     if (exy && ez >= 0 && ez < nelz) pE = __ldg(E + eofs + ez * EP);
+  };
+  // the epilogue operands of plane z
+  auto fetch_out = [&](int z) {
+    if (!Sg::kIn && Sg::kArrays > 0 && own && z >= zs && z < ze) {
+      const int64_t i = 3 * ((int64_t)nofs + (int64_t)z * NP);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (Sg::kB) copy_async(slot_at(Sg::kSlotB, z, ty) + c, args.b + i + c);
+        if (Sg::kD) copy_async(slot_at(Sg::kSlotD, z, ty) + c, args.dinv + i + c);
+        if (Sg::kY) copy_async(slot_at(Sg::kSlotY, z, ty) + c, args.y2 + i + c);
+      }
+    }
   };
 
   T FA[4][3], FB[4][3], CA[4][3], CB[4][3], les[3], led[3];
@@ -233,6 +290,21 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
                   T(&top)[4][3]) {
     T cu[3], cq[3];
     const unsigned f = pf;
+    if (Sg::kArrays > 0) copy_wait();   // issued one plane ago, by this thread for itself
+    if (Sg::kIn) {
+      const T *sb = slot_at(Sg::kSlotB, p, ty), *sd = slot_at(Sg::kSlotD, p, ty);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) pu[c] = args.invtheta * (sd[c] * sb[c]);
+      if (lastrow) {
+        const T *qb = slot_at(Sg::kSlotB, p, TY), *qd = slot_at(Sg::kSlotD, p, TY);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) pq[c] = args.invtheta * (qd[c] * qb[c]);
+      }
+    } else if (Sg::kU) {
+      T *r = ring_at(p);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) r[c] = pu[c];
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       cu[c] = ((f >> c) & 1u) ? T(0) : pu[c];
@@ -241,6 +313,7 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     const T Ee = pE;
     fpipe = (fpipe << 8) | f;
     if (p + 1 <= ze) fetch(p + 1);
+    fetch_out(p - 1);
     const int rb = (p & 1) * kRows, rb1 = kRows - rb;   // this / the other buffer
 
     // ---- x-edges of plane p (s = u(x+1) + u(x), d = u(x+1) - u(x)) and
@@ -291,15 +364,25 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
         val[c] = (es - ed) + left;
       }
       if (own) {
-        const int64_t n = nofs + (int64_t)(p - 2) * NP;
+        const int64_t i = 3 * (nofs + (int64_t)(p - 2) * NP);
         const unsigned fo = (fpipe >> 16) & 0xffu;
+        const T *sb = slot_at(Sg::kSlotB, p - 2, ty), *sd = slot_at(Sg::kSlotD, p - 2, ty),
+                *sy = slot_at(Sg::kSlotY, p - 2, ty), *su = ring_at(p - 2);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           const bool fixed = (fo >> c) & 1u;
+          const T bi = Sg::kB ? sb[c] : T(0), di = Sg::kD ? sd[c] : T(0),
+                  yi = Sg::kY ? sy[c] : T(0);
           // the input is needed on fixed dofs (identity rows) and by the
           // Chebyshev epilogues
-          const T uv = (kNeedU || fixed) ? input_value<T, IN>(args, 3 * n + c) : T(0);
-          finish_dof<T, OUT>(args, 3 * n + c, fixed ? uv : val[c], uv);
+          T uv = T(0);
+          if (Sg::kIn)
+            uv = args.invtheta * (di * bi);
+          else if (Sg::kU)
+            uv = su[c];
+          else if (fixed)
+            uv = __ldg(args.u + i + c);
+          sym_out_v<T, OUT>(args, i + c, fixed ? uv : val[c], uv, bi, di, yi);
         }
       }
     }
@@ -363,19 +446,19 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
 
 constexpr int kTY = 8;
 
-template <typename T>
-size_t staged_smem() {
-  return 4 * Six<T>::bytes_per_row() * (kTY + 1);
+template <typename T, int IN, int OUT>
+constexpr size_t staged_smem() {
+  return (kTY + 1) * (4 * Six<T>::bytes_per_row() + Staged<IN, OUT>::planes() * 96 * sizeof(T));
 }
 
 template <typename T, int IN, int OUT>
 void set_smem_attr() {
   cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, false>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)staged_smem<T>());
+                       (int)staged_smem<T, IN, OUT>());
   cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, true>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)staged_smem<T>());
+                       (int)staged_smem<T, IN, OUT>());
 }
 
 // grid of the staged kernel: 30 x (kTY-1) owned node columns per CTA, and z
@@ -399,7 +482,7 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
     int per_sm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true>, 32 * kTY,
-        staged_smem<T>());
+        staged_smem<T, IN_CHEB, OUT_CHEB2>());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     slots_cache[dev] = std::max(1, per_sm) * std::max(1, sms);
     attr_set |= 1ull << dev;
@@ -433,10 +516,10 @@ void launch_mode(const Ctx &c, const T *E, const ApplyArgs<T> &args_in,
       sizeof(T) == 8 ? (const void *)&c.kh64 : (const void *)&c.kh32);
   count_launch();
   if (nb == 1)
-    k_apply_staged<T, kTY, IN, OUT, false><<<grid, dim3(32, kTY), staged_smem<T>(), s>>>(
+    k_apply_staged<T, kTY, IN, OUT, false><<<grid, dim3(32, kTY), staged_smem<T, IN, OUT>(), s>>>(
         c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh);
   else
-    k_apply_staged<T, kTY, IN, OUT, true><<<grid, dim3(32, kTY), staged_smem<T>(), s>>>(
+    k_apply_staged<T, kTY, IN, OUT, true><<<grid, dim3(32, kTY), staged_smem<T, IN, OUT>(), s>>>(
         c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh);
 }
 

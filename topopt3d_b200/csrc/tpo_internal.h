@@ -316,7 +316,7 @@ void launch_apply_fine(const Ctx &c, const T *E, const T *u, const T *b, T *y,
                        cudaStream_t s, int nb = 1);
 
 // fused fine-level variants: how the input is formed and what the epilogue
-// writes (kernels_apply_staged.cu, finish_dof)
+// writes (sym_out_v, fused_out.cuh)
 enum { IN_U = 0, IN_CHEB = 1 };
 enum { OUT_Y = 0, OUT_RESID = 1, OUT_CHEB2 = 2, OUT_POST0 = 3, OUT_POST1 = 4 };
 
