@@ -45,3 +45,39 @@ def test_coarsest_inverse_is_the_inverse(T, nel):
     t.apply(np.eye(n).reshape(-1), K, nrhs=n)
     w = np.linalg.eigvalsh(K.reshape(n, n))
     assert np.linalg.norm(y - r) <= n * 1.1e-16 * w[-1] / w[0] * np.linalg.norm(r)
+
+
+# the eigensolver's Gram and recombination kernels: blocks of 8, 40 / 72
+# (Gram tiles) and 8 .. 64 output columns, fewer rows than a chunk of 64 and
+# a partial last one (81, 648 and 1,155 dof), odd and even row counts
+@pytest.mark.parametrize("nel,levels,nev,block", [((2, 2, 2), 1, 1, 3), ((5, 5, 5), 1, 2, 4),
+                                                  ((10, 6, 4), 2, 3, 7), ((10, 6, 4), 2, 3, 10),
+                                                  ((10, 6, 4), 2, 6, 13),
+                                                  ((10, 6, 4), 2, 4, 20),
+                                                  ((10, 6, 4), 2, 8, 32)])
+def test_eigensolver_block_sizes(T, nel, levels, nev, block):
+    """The lowest lumped-mass frequencies against a dense generalized
+    eigensolve of the operator's own columns: a residual of tol leaves a
+    relative eigenvalue error of tol^2 cond, below rounding (n u cond)."""
+    t = make(T, nel, levels)
+    n = 3 * t.nNode
+    lam, _ = t.frequency(nev, 1.0, block=block, tol=1e-9, maxit=2000)
+    assert t.last_eig["rc"] == 0
+    K = np.zeros(n * n)
+    t.apply(np.eye(n).reshape(-1), K, nrhs=n)
+    K = K.reshape(n, n)
+    # DiagMassFnc: element volume x density / 24 at each of its nodes, 1e-8
+    # at fixed dofs
+    nx, ny, nz = nel
+    rho = t.rho.reshape(nz, ny, nx)
+    m = np.zeros((nz + 1, ny + 1, nx + 1))
+    for c in range(8):
+        i, j, k = c & 1, (c >> 1) & 1, c >> 2
+        m[k:k + nz, j:j + ny, i:i + nx] += rho / 24.0
+    fm, _ = t.get_bc()
+    free = np.array([not (fm[d // 3] >> (d % 3)) & 1 for d in range(n)])
+    M = np.repeat(m.reshape(-1), 3)[free]
+    import scipy.linalg as sl
+    ref = sl.eigh(np.diag(M), K[np.ix_(free, free)], eigvals_only=True)[::-1]
+    w = np.linalg.eigvalsh(K)
+    assert np.allclose(lam, ref[:lam.size], rtol=n * 1.1e-16 * w[-1] / w[0] + 1e-13, atol=0)
