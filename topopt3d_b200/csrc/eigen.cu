@@ -260,7 +260,7 @@ int buckling(Ctx &c, const tpo_eig_opts &o, double *lambda, double *phi,
       count_launch();
       k_diag_apply<<<grid_for(n * m, 256), 256, 0, s>>>(n, m, adiag, V, AV);
     } else {
-      launch_ks_apply(c, V, AV, m);
+      launch_ks_apply(c, V, AV, m, true);   // every block is masked
     }
     for (int j0 = 0; j0 < m;) {
       const int nb = std::min(m - j0, kMaxBatch);

@@ -501,7 +501,7 @@ void launch_freq_gradient(const Ctx &c, const double *phi, int64_t ld, int nterm
 void launch_bk_gradient(const Ctx &c, const double *phi, const double *v, int64_t ld,
                         int nev, const BkCoef &coef, double *g, cudaStream_t s);
 // y = Ks u for nb columns (stride 3 nn), on c.stream
-void launch_ks_apply(const Ctx &c, const double *u, double *y, int nb);
+void launch_ks_apply(const Ctx &c, const double *u, double *y, int nb, bool masked = false);
 void launch_sensitivity(const Ctx &c, const double *U, double *dc,
                         cudaStream_t s);
 void launch_oc_step(const Ctx &c, int64_t n, double *x, const double *xold,
