@@ -225,8 +225,11 @@ int alloc_solver(Ctx &c) {
         A(v.H32, 126 * ((v.nn + 31) / 32) * 32);   // tiles of 32 nodes (kernels_mg.cu)
       }
       if (l >= c.ps && l + 1 < c.L) {
-        A(v.A64, 243 * v.nn);
-        A(v.A32, 243 * v.nn);
+        const int ctas = tpo::coarse_ctas(c.device);
+        int npc = 0, npcp = 0;
+        tpo::coarse_slab(v.nn, ctas, &npc, &npcp);
+        A(v.A64, (size_t)ctas * 243 * npcp);
+        A(v.A32, (size_t)ctas * 243 * npcp);
       }
     }
   }

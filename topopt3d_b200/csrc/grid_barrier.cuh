@@ -46,4 +46,40 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, double *fault,
   return ok != 0;
 }
 
+// The same barrier for a kernel that passes many: the block remembers which
+// way bit 31 points (`sense`, read before its first arrival, when it cannot
+// flip yet), so the arrival is a reduction without a return value and the
+// first poll follows it at once, one L2 round trip less per barrier (about
+// 0.4 us of 1.6 us).  Thread 0's value of *sense is the one used.
+__device__ __forceinline__ unsigned int grid_barrier_sense(const unsigned int *bar) {
+  unsigned int cur = 0;
+  if (threadIdx.x == 0)
+    asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(cur) : "l"(bar) : "memory");
+  return cur & 0x80000000u;
+}
+__device__ __forceinline__ bool grid_barrier_red(unsigned int *bar, double *fault,
+                                                 unsigned int *sense,
+                                                 int max_polls = kBarrierPolls) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned int add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
+    asm volatile("red.add.release.gpu.u32 [%0], %1;" ::"l"(bar), "r"(add) : "memory");
+    unsigned int cur;
+    int polls = 0;
+    ok = 1;
+    do {
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(cur) : "l"(bar) : "memory");
+      if (++polls > max_polls) {
+        ok = 0;
+        *(volatile double *)fault = 1.0;
+        break;
+      }
+    } while (((*sense ^ cur) & 0x80000000u) == 0u);
+    *sense ^= 0x80000000u;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
 }  // namespace tpo

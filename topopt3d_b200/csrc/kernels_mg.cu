@@ -498,11 +498,12 @@ __global__ void k_stencil_diag(int64_t nn, const double *__restrict__ S,
   }
 }
 
-// b_c = P^T r_f for nb columns (fine stride 3 nnf, coarse stride 3 nnc)
-template <typename T>
+// b_c = P^T r_f for nb columns (fine stride 3 nnf, coarse stride 3 nnc);
+// COMP: b_c component by component, with the first Chebyshev direction
+template <typename T, bool COMP>
 __global__ void k_restrict(int fx, int fy, int fz, int cx, int cy, int cz,
                            const T *__restrict__ rf, T *__restrict__ bc,
-                           int nb) {
+                           const CompLevel<T> comp, int nb) {
   const int64_t nnc = (int64_t)cx * cy * cz, nnf = (int64_t)fx * fy * fz;
   for (int64_t I = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; I < nnc;
        I += (int64_t)gridDim.x * blockDim.x) {
@@ -511,15 +512,21 @@ __global__ void k_restrict(int fx, int fy, int fz, int cx, int cy, int cz,
       T s[3];
       restrict_node(fx, fy, fz, ix, iy, iz, rf + col * 3 * nnf, s);
       T *o = bc + col * 3 * nnc;
-      o[3 * I] = s[0];
-      o[3 * I + 1] = s[1];
-      o[3 * I + 2] = s[2];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if (COMP) {
+          o[c * nnc + I] = s[c];
+          comp.d0[(3 * col + c) * nnc + I] = comp.inv_theta * (comp.dinv[3 * I + c] * s[c]);
+        } else {
+          o[3 * I + c] = s[c];
+        }
+      }
     }
   }
 }
 
-// x_f += P x_c for nb columns
-template <typename T>
+// x_f += P x_c for nb columns; COMP: x_c component by component
+template <typename T, bool COMP>
 __global__ void k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz,
                               const T *__restrict__ xc, T *__restrict__ xf,
                               int nb) {
@@ -529,7 +536,8 @@ __global__ void k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz,
     const int gx = f % fx, gy = (f / fx) % fy, gz = f / ((int64_t)fx * fy);
     for (int col = 0; col < nb; ++col) {
       T s[3];
-      prolong_node(fx, fy, fz, cx, cy, cz, gx, gy, gz, xc + col * 3 * nnc, s);
+      prolong_node(fx, fy, fz, cx, cy, cz, gx, gy, gz, xc + col * 3 * nnc, COMP ? 1 : 3,
+                   COMP ? nnc : 1, s);
       T *o = xf + col * 3 * nnf;
       o[3 * f] += s[0];
       o[3 * f + 1] += s[1];
@@ -755,54 +763,42 @@ void launch_stencil_diag(const Level &v, const double *S, double *dinv64,
 }
 
 template <typename T>
-void launch_restrict(const Level &fine, const Level &coarse, const T *rf,
-                     T *bc, cudaStream_t s, int nb) {
+void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *bc,
+                     const CompLevel<T> *comp, cudaStream_t s, int nb) {
   count_launch();
-  k_restrict<T><<<grid_for(coarse.nn, 128), 128, 0, s>>>(
-      fine.dims[0], fine.dims[1], fine.dims[2], coarse.dims[0], coarse.dims[1],
-      coarse.dims[2], rf, bc, nb);
+  const int g = grid_for(coarse.nn, 128);
+  if (comp)
+    k_restrict<T, true><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
+                                          coarse.dims[0], coarse.dims[1], coarse.dims[2], rf, bc,
+                                          *comp, nb);
+  else
+    k_restrict<T, false><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
+                                           coarse.dims[0], coarse.dims[1], coarse.dims[2], rf, bc,
+                                           CompLevel<T>{}, nb);
 }
-template void launch_restrict<double>(const Level &, const Level &,
-                                      const double *, double *, cudaStream_t,
-                                      int);
-template void launch_restrict<float>(const Level &, const Level &,
-                                     const float *, float *, cudaStream_t, int);
+template void launch_restrict<double>(const Level &, const Level &, const double *, double *,
+                                      const CompLevel<double> *, cudaStream_t, int);
+template void launch_restrict<float>(const Level &, const Level &, const float *, float *,
+                                     const CompLevel<float> *, cudaStream_t, int);
 
 template <typename T>
-void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc,
-                        T *xf, cudaStream_t s, int nb) {
+void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc, T *xf, bool comp,
+                        cudaStream_t s, int nb) {
   count_launch();
-  k_prolong_add<T><<<grid_for(fine.nn, 128), 128, 0, s>>>(
-      fine.dims[0], fine.dims[1], fine.dims[2], coarse.dims[0], coarse.dims[1],
-      coarse.dims[2], xc, xf, nb);
+  const int g = grid_for(fine.nn, 128);
+  if (comp)
+    k_prolong_add<T, true><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
+                                             coarse.dims[0], coarse.dims[1], coarse.dims[2], xc,
+                                             xf, nb);
+  else
+    k_prolong_add<T, false><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
+                                              coarse.dims[0], coarse.dims[1], coarse.dims[2], xc,
+                                              xf, nb);
 }
-template void launch_prolong_add<double>(const Level &, const Level &,
-                                         const double *, double *,
-                                         cudaStream_t, int);
-template void launch_prolong_add<float>(const Level &, const Level &,
-                                        const float *, float *, cudaStream_t,
-                                        int);
-
-namespace {
-__global__ void k_soa_to_aos(int64_t nn, const double *__restrict__ S,
-                             double *__restrict__ A64, float *__restrict__ A32) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nn * 243;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = t / 243;
-    const int w = (int)(t - n * 243);   // (3r+s)*27 + nb
-    const int q = (w % 27) * 9 + w / 27;
-    const double v = S[(int64_t)q * nn + n];
-    A64[t] = v;
-    A32[t] = static_cast<float>(v);
-  }
-}
-}  // namespace
-
-void launch_soa_to_aos(int64_t nn, const double *S, double *A64, float *A32,
-                       cudaStream_t s) {
-  count_launch();
-  k_soa_to_aos<<<grid_for(nn * 243, 256), 256, 0, s>>>(nn, S, A64, A32);
-}
+template void launch_prolong_add<double>(const Level &, const Level &, const double *, double *,
+                                         bool, cudaStream_t, int);
+template void launch_prolong_add<float>(const Level &, const Level &, const float *, float *,
+                                        bool, cudaStream_t, int);
 
 template <typename T>
 void launch_coarse_gemv(int64_t n, const double *Ainv, const T *b, T *x,

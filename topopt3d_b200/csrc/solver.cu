@@ -93,7 +93,8 @@ CoarseCycle<T> coarse_cycle_params(Ctx &c, const tpo_solve_opts &o) {
     LV<T> w = lv(v, (T *)nullptr);
     CoarseLevel<T> &L = P.lev[i];
     for (int d = 0; d < 3; ++d) L.dims[d] = v.dims[d];
-    L.nn = v.nn;
+    L.nn = (int)v.nn;
+    coarse_slab(v.nn, coarse_ctas(c.device), &L.npc, &L.npcp);
     L.A = (sizeof(T) == 8) ? reinterpret_cast<const T *>(v.A64)
                            : reinterpret_cast<const T *>(v.A32);
     L.dinv = w.dinv;
@@ -130,6 +131,28 @@ CoarseCycle<T> coarse_cycle_params(Ctx &c, const tpo_solve_opts &o) {
   P.bar = c.gbar;
   P.fault = c.scal + kSlotFault;
   return P;
+}
+
+// the transfers between level l and l + 1: the top level of the persistent
+// kernel keeps its vectors component by component
+bool comp_level(const Ctx &c, int l) { return l == c.ps && l + 1 < c.L; }
+
+template <typename T>
+void restrict_to(Ctx &c, int l, const T *r, const tpo_solve_opts &o, cudaStream_t s, int nb) {
+  Level &v = c.lev[l], &cv = c.lev[l + 1];
+  LV<T> cw = lv(cv, (T *)nullptr);
+  if (comp_level(c, l + 1)) {
+    const CompLevel<T> top{cw.dinv, cw.d, static_cast<T>(cheb_of(cv.lam, o).inv_theta)};
+    launch_restrict<T>(v, cv, r, cw.b, &top, s, nb);
+  } else {
+    launch_restrict<T>(v, cv, r, cw.b, nullptr, s, nb);
+  }
+}
+
+template <typename T>
+void prolong_from(Ctx &c, int l, T *x, cudaStream_t s, int nb) {
+  Level &v = c.lev[l], &cv = c.lev[l + 1];
+  launch_prolong_add<T>(v, cv, lv(cv, (T *)nullptr).x, x, comp_level(c, l + 1), s, nb);
 }
 
 template <typename T>
@@ -186,9 +209,9 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
     fused(IN_U, OUT_RESID);
     Level &cv = c.lev[l + 1];
     LV<T> cw = lv(cv, (T *)nullptr);
-    launch_restrict<T>(v, cv, w.a, cw.b, s, nb);
+    restrict_to<T>(c, l, w.a, o, s, nb);
     vcycle_rec<T>(c, l + 1, cw.b, cw.x, o, s, nb);
-    launch_prolong_add<T>(v, cv, cw.x, x, s, nb);
+    prolong_from<T>(c, l, x, s, nb);
     a.u = x;                                                   // post-smooth
     a.y = w.d;
     a.y2 = w.r;
@@ -212,9 +235,9 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
   level_apply<T>(c, l, x, b, w.a, s, nb);
   Level &cv = c.lev[l + 1];
   LV<T> cw = lv(cv, (T *)nullptr);
-  launch_restrict<T>(v, cv, w.a, cw.b, s, nb);
+  restrict_to<T>(c, l, w.a, o, s, nb);
   vcycle_rec<T>(c, l + 1, cw.b, cw.x, o, s, nb);
-  launch_prolong_add<T>(v, cv, cw.x, x, s, nb);
+  prolong_from<T>(c, l, x, s, nb);
   // post-smoothing from the corrected x
   level_apply<T>(c, l, x, b, w.r, s, nb);
   launch_cheb_init<T>(n, w.dinv, b, w.r, w.d, x, ch.inv_theta, false, s, nb);
@@ -646,8 +669,8 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
                              c.lev[l + 1].H32, s);
     }
     if (l + 1 >= c.ps && l + 1 < c.L - 1)
-      launch_soa_to_aos(c.lev[l + 1].nn, c.lev[l + 1].S64, c.lev[l + 1].A64,
-                        c.lev[l + 1].A32, s);
+      launch_coarse_slabs(c.lev[l + 1], coarse_ctas(c.device), c.lev[l + 1].S64,
+                          c.lev[l + 1].A64, c.lev[l + 1].A32, s);
     if (int rc = level_ready(l + 1)) {
       join();
       return rc;

@@ -73,7 +73,7 @@ struct Level {
   // S[(nb*9 + 3r + s) * nn + node], nb = (dk+1)*9 + (dj+1)*3 + (di+1)
   double *S64 = nullptr;
   float *S32 = nullptr;
-  // node-major copies A[n*243 + (3r + s)*27 + nb] for the persistent kernel
+  // the same by CTA of the persistent kernel (launch_coarse_slabs)
   double *A64 = nullptr;
   float *A32 = nullptr;
   // symmetric half (centre + 13 forward blocks) for the levels between the
@@ -374,16 +374,30 @@ size_t galerkin_dims_scratch(const Level &fine);
 int launch_galerkin_fine(Ctx &c, double *Sc, cudaStream_t s);
 void launch_stencil_diag(const Level &v, const double *S, double *dinv64,
                          float *dinv32, cudaStream_t s);
+// The top level of the persistent kernel keeps its vectors component by
+// component (coarse.h); a restriction into it also writes the first
+// Chebyshev direction d0 = inv_theta D^-1 b.
 template <typename T>
-void launch_restrict(const Level &fine, const Level &coarse, const T *rf,
-                     T *bc, cudaStream_t s, int nb = 1);
+struct CompLevel {
+  const T *dinv;
+  T *d0;
+  T inv_theta;
+};
+// bc = P^T rf; comp: bc (and d0) component by component
 template <typename T>
-void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc,
-                        T *xf, cudaStream_t s, int nb = 1);
-// stencil SoA S[(nb*9 + 3r+s)*nn + n] -> node-major A[n*243 + (3r+s)*27 + nb]
-// (FP64 and an FP32 copy)
-void launch_soa_to_aos(int64_t nn, const double *S, double *A64, float *A32,
-                       cudaStream_t s);
+void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *bc,
+                     const CompLevel<T> *comp, cudaStream_t s, int nb = 1);
+// xf += P xc; comp: xc component by component
+template <typename T>
+void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc, T *xf, bool comp,
+                        cudaStream_t s, int nb = 1);
+// the persistent coarse cycle (kernels_coarse.cu): its CTAs (one per SM of
+// the device), the nodes of a level each owns, and the stencil SoA S[(nb*9 +
+// 3r+s)*nn + n] by CTA, A[(cta * 243 + nb*9 + 3r+s) * npcp + i], FP64 and FP32
+int coarse_ctas(int dev);
+void coarse_slab(int64_t nn, int ctas, int *npc, int *npcp);
+void launch_coarse_slabs(const Level &v, int ctas, const double *S, double *A64, float *A32,
+                         cudaStream_t s);
 // Ainv (n x n) = the inverse of the level's SPD stencil operator S
 // (kernels_coarse_inv.cu); work holds coarse_inverse_work(plan) doubles;
 // *info becomes the index + 1 of the first dof whose pivot is not positive

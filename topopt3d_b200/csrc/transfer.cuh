@@ -59,12 +59,13 @@ __device__ __forceinline__ void restrict_node(int fx, int fy, int fz, int ix,
   s[2] = s2;
 }
 
-// sum over the coarse nodes I around fine node (gx,gy,gz) of P(f,I) x_I
+// sum over the coarse nodes I around fine node (gx,gy,gz) of P(f,I) x_I;
+// component c of node I at xc[I * sn + c * sc]
 template <typename T>
 __device__ __forceinline__ void prolong_node(int fx, int fy, int fz, int cx,
                                              int cy, int cz, int gx, int gy,
                                              int gz, const T *__restrict__ xc,
-                                             T s[3]) {
+                                             int64_t sn, int64_t sc, T s[3]) {
   const int g[3] = {gx, gy, gz}, F[3] = {fx, fy, fz}, Cn[3] = {cx, cy, cz};
   int c0[3], c1[3];
   double w0[3], w1[3];
@@ -85,9 +86,9 @@ __device__ __forceinline__ void prolong_node(int fx, int fy, int fz, int cx,
                                (az ? w1[2] : w0[2]));
     const int64_t I = ((int64_t)(az ? c1[2] : c0[2]) * cy + (ay ? c1[1] : c0[1])) * cx +
                       (ax ? c1[0] : c0[0]);
-    s0 += w * xc[3 * I];
-    s1 += w * xc[3 * I + 1];
-    s2 += w * xc[3 * I + 2];
+    s0 += w * xc[I * sn];
+    s1 += w * xc[I * sn + sc];
+    s2 += w * xc[I * sn + 2 * sc];
   }
   s[0] = s0;
   s[1] = s1;
