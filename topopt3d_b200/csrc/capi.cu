@@ -221,7 +221,7 @@ int alloc_solver(Ctx &c) {
     if (l > 0) {
       A(v.S64, 243 * v.nn);
       if (l < c.ps) {
-        A(v.H64, 126 * v.nn);
+        v.H64 = v.S64 + 117 * v.nn;
         A(v.H32, 126 * ((v.nn + 31) / 32) * 32);   // tiles of 32 nodes (kernels_mg.cu)
       }
       if (l >= c.ps && l + 1 < c.L) {
@@ -255,7 +255,7 @@ void free_all(Ctx &c) {
   free_columns(c);
   for (tpo::Level &v : c.lev) {
     dfree(v.S64); dfree(v.S32); dfree(v.dinv64); dfree(v.dinv32);
-    dfree(v.A64); dfree(v.A32); dfree(v.H64); dfree(v.H32);
+    dfree(v.A64); dfree(v.A32); v.H64 = nullptr; dfree(v.H32);
   }
   dfree(c.fix); dfree(c.idm); dfree(c.F); dfree(c.U); dfree(c.x); dfree(c.rho);
   dfree(c.E64); dfree(c.dEdz); dfree(c.E32); dfree(c.S0); dfree(c.K0lex);

@@ -3,7 +3,8 @@
 // They match the fine-level kernel's (kernels_apply_staged.cu):
 // IN_U reads u, IN_CHEB forms the Chebyshev start invtheta D^-1 b on the
 // fly; OUT_Y / OUT_RESID / OUT_CHEB2 / OUT_POST0 / OUT_POST1 write Au,
-// b - Au or the fused Chebyshev(2) updates.
+// b - Au or the fused Chebyshev(2) updates, OUT_SCALE D^-1 Au (a step of the
+// power iteration).
 #pragma once
 
 #include "tpo_internal.h"
@@ -32,6 +33,8 @@ __device__ __forceinline__ void sym_out_v(const ApplyArgs<T> &a, I i, T Au, T u,
     const T d0 = a.invtheta * (di * (bi - Au));
     a.y[i] = d0;
     a.y2[i] = u + d0;
+  } else if (OUT == OUT_SCALE) {
+    a.y[i] = Au * di;
   } else {   // OUT_POST1
     const T r1 = a.theta * u - di * Au;
     a.y[i] = y2i + (a.c1 * u + a.c2 * r1);
@@ -41,7 +44,8 @@ __device__ __forceinline__ void sym_out_v(const ApplyArgs<T> &a, I i, T Au, T u,
 template <int OUT>
 struct OutNeeds {
   static constexpr bool b = OUT == OUT_RESID || OUT == OUT_CHEB2 || OUT == OUT_POST0;
-  static constexpr bool dinv = OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1;
+  static constexpr bool dinv = OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1 ||
+                               OUT == OUT_SCALE;
   static constexpr bool y2 = OUT == OUT_POST1;
 };
 

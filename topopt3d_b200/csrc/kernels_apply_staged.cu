@@ -56,6 +56,7 @@ constexpr int kLanesOut = 30;   // written nodes per tile row
 //             y = d0, y2 = u + d0
 //   OUT_POST1 second step, input d0 = u (so r0 = theta d0):
 //             d1 = c1 d0 + c2 (theta d0 - dinv Au); y = x1 + d1 (x1 = y2)
+//   OUT_SCALE y = dinv Au
 // (sym_out_v, fused_out.cuh)
 
 // Operands that a thread reads for its own node only -- b, dinv, y2 of the
@@ -479,6 +480,7 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
     set_smem_attr<T, IN_CHEB, OUT_CHEB2>();
     set_smem_attr<T, IN_U, OUT_POST0>();
     set_smem_attr<T, IN_U, OUT_POST1>();
+    set_smem_attr<T, IN_U, OUT_SCALE>();
     int per_sm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true>, 32 * kTY,
@@ -549,6 +551,8 @@ void launch_apply_fused(const Ctx &c, const T *E, int in, int out,
     launch_mode<T, IN_U, OUT_POST1>(c, E, args, s, nb);
   else if (in == IN_U && out == OUT_RESID)
     launch_mode<T, IN_U, OUT_RESID>(c, E, args, s, nb);
+  else if (in == IN_U && out == OUT_SCALE)
+    launch_mode<T, IN_U, OUT_SCALE>(c, E, args, s, nb);
   else
     launch_mode<T, IN_U, OUT_Y>(c, E, args, s, nb);
 }

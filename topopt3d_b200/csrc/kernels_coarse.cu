@@ -42,7 +42,6 @@
 // stencil from DRAM 17 k, the inverse (29 MB) 14 k, the other phases 2 - 9 k.
 #include "coarse.h"
 #include "grid_barrier.cuh"
-#include "transfer.cuh"
 #include "umma.cuh"
 
 namespace tpo {

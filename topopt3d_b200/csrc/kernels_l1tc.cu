@@ -400,7 +400,9 @@ __global__ void __launch_bounds__(kThreads, 2)
         pd[d] = ((OutNeeds<OUT>::dinv || IN == IN_CHEB) && own) ? a.dinv[gi + d] : 0.0f;
         p2[d] = (OutNeeds<OUT>::y2 && own) ? a.y2[gi + d] : 0.0f;
         pc[d] = (corr && own) ? p.cval[gi + d] : 0.0f;
-        pu[d] = (IN == IN_U && OUT != OUT_Y && OUT != OUT_RESID && own) ? a.u[gi + d] : 0.0f;
+        pu[d] = (IN == IN_U && OUT != OUT_Y && OUT != OUT_RESID && OUT != OUT_SCALE && own)
+                    ? a.u[gi + d]
+                    : 0.0f;
       }
       if (more) moduli(k + 1, Enext);
       const bool ok = umma::mbar_wait(&mbar[b], (uint32_t)((it >> 1) & 1), kWaitPolls);
@@ -623,6 +625,8 @@ void launch_l1tc(const Ctx &c, int in, int out, const ApplyArgs<float> &a, cudaS
     launch_mode<IN_U, OUT_POST1>(p, grid, a, pdl, s);
   else if (out == OUT_RESID)
     launch_mode<IN_U, OUT_RESID>(p, grid, a, pdl, s);
+  else if (out == OUT_SCALE)
+    launch_mode<IN_U, OUT_SCALE>(p, grid, a, pdl, s);
   else
     launch_mode<IN_U, OUT_Y>(p, grid, a, pdl, s);
 }

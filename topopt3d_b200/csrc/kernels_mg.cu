@@ -16,7 +16,6 @@
 #include <algorithm>
 
 #include "tpo_internal.h"
-#include "transfer.cuh"
 #include "fused_out.cuh"
 
 namespace tpo {
@@ -82,122 +81,256 @@ __global__ void k_coarse_elem_flags(int nelx, int nely, int nelz,
   }
 }
 
-// general path, one thread per (flagged coarse element, ln, lm): the 3x3
-// block sum_{fine e in E} E_e sum_{p,q} w(p->ln) w(q->lm) (M K0 M)_pq with
-// the interpolation weights of pw1 and the identity-dof masks
-__global__ void k_galerkin_general(int nelx, int nely, int nelz, int nslots,
-                                   const double *__restrict__ E,
-                                   const uint8_t *__restrict__ idm,
-                                   const int *__restrict__ slot_elem,
-                                   const double *__restrict__ K0lex,
-                                   double *__restrict__ G) {
+// general path: the 3x3 block (ln, lm) of a flagged coarse element,
+// sum_{fine e in E} E_e sum_{p,q} w(p->ln) w(q->lm) (M K0 M)_pq with the
+// interpolation weights of pw1 and the identity-dof masks.  A CTA takes one
+// (ln, lm) of 32 elements, a warp one of their fine elements i, so that which
+// of the 64 corner pairs have a weight is the same for a warp and the others
+// are skipped (a thread per block, or lanes of different i, went through all:
+// 184 and 241 us for the 2,304 elements of a 192x96x96 cantilever's face; now
+// 121 us).  A fine element without identity dofs uses its fixed block.  The
+// eight sums are added in order.
+__global__ void __launch_bounds__(256)
+    k_galerkin_general(int nelx, int nely, int nelz, int nslots, const double *__restrict__ E,
+                       const uint8_t *__restrict__ idm, const int *__restrict__ slot_elem,
+                       const double *__restrict__ K0lex, const double *__restrict__ GMi,
+                       double *__restrict__ G) {
+  __shared__ double K0[576];
+  __shared__ double sum[8][9][32];
+  for (int e = threadIdx.x; e < 576; e += 256) K0[e] = K0lex[e];
+  __syncthreads();
   const int fx = nelx + 1, fy = nely + 1, fz = nelz + 1;
   const int ncx = (nelx + 1) / 2, ncy = (nely + 1) / 2;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 64 * (int64_t)nslots;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int sl = (int)(t / 64), pr = (int)(t % 64), ln = pr / 8, lm = pr % 8;
+  const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
+  const int ln = blockIdx.y / 8, lm = blockIdx.y % 8;
+  const int sl = blockIdx.x * 32 + lane;
+  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  if (sl < nslots) {
     const int ce = slot_elem[sl];
     const int EI = ce % ncx, EJ = (ce / ncx) % ncy, EK = ce / (ncx * ncy);
-    // coarse corner coordinates (the far ones may not exist: pw1 gives 0)
-    const int ix = EI + (ln & 1), iy = EJ + ((ln >> 1) & 1), iz = EK + ((ln >> 2) & 1);
-    const int jx = EI + (lm & 1), jy = EJ + ((lm >> 1) & 1), jz = EK + ((lm >> 2) & 1);
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = 0; i < 8; ++i) {
-      const int ex = 2 * EI + (i & 1), ey = 2 * EJ + ((i >> 1) & 1), ez = 2 * EK + ((i >> 2) & 1);
-      if (ex >= nelx || ey >= nely || ez >= nelz) continue;
+    const int ex = 2 * EI + (i & 1), ey = 2 * EJ + ((i >> 1) & 1), ez = 2 * EK + ((i >> 2) & 1);
+    if (ex < nelx && ey < nely && ez < nelz) {
       const double Ee = E[((int64_t)ez * nely + ey) * nelx + ex];
-      double wn[8], wm[8];
+      // 1-D weights of the two corners of the fine element per dimension
+      // (zero where a far coarse corner does not exist)
+      const int f0[3] = {ex, ey, ez}, C[3] = {EI, EJ, EK}, N[3] = {fx, fy, fz};
+      double wn[3][2], wm[3][2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          wn[d][t] = pw1(f0[d] + t, C[d] + ((ln >> d) & 1), N[d]);
+          wm[d][t] = pw1(f0[d] + t, C[d] + ((lm >> d) & 1), N[d]);
+        }
       unsigned msk[8];
 #pragma unroll
-      for (int p = 0; p < 8; ++p) {
-        const int gx = ex + (p & 1), gy = ey + ((p >> 1) & 1), gz = ez + ((p >> 2) & 1);
-        wn[p] = pw1(gx, ix, fx) * pw1(gy, iy, fy) * pw1(gz, iz, fz);
-        wm[p] = pw1(gx, jx, fx) * pw1(gy, jy, fy) * pw1(gz, jz, fz);
-        msk[p] = idm[((int64_t)gz * fy + gy) * fx + gx];
+      for (int p = 0; p < 8; ++p)
+        msk[p] = idm[((int64_t)(ez + (p >> 2)) * fy + ey + ((p >> 1) & 1)) * fx + ex + (p & 1)];
+      // no identity dof here and all coarse corners there: the fixed block
+      const bool plain = !(msk[0] | msk[1] | msk[2] | msk[3] | msk[4] | msk[5] | msk[6] | msk[7]) &&
+                         2 * EI + 2 <= nelx && 2 * EJ + 2 <= nely && 2 * EK + 2 <= nelz;
+      if (plain) {
+        const double *m = GMi + ((i * 8 + ln) * 8 + lm) * 9;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc[q] = Ee * m[q];
       }
+      // corner p of fine element i lies at t = i + p per dimension from the
+      // coarse element's origin: no weight on ln when |t - 2 ln| = 2
+      auto off = [&](int p, int l) {
+        bool z = false;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int t = ((i >> d) & 1) + ((p >> d) & 1) - 2 * ((l >> d) & 1);
+          z |= t == 2 || t == -2;
+        }
+        return z;
+      };
+#pragma unroll
       for (int p = 0; p < 8; ++p) {
-        if (wn[p] == 0.0) continue;
+        if (plain || off(p, ln)) continue;
+        const double wp = Ee * (wn[0][p & 1] * wn[1][(p >> 1) & 1] * wn[2][p >> 2]);
+#pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const double w = Ee * wn[p] * wm[q];
-          if (w == 0.0) continue;
-          const double *k0 = K0lex + 24 * (3 * p) + 3 * q;
-          for (int r = 0; r < 3; ++r) {
-            if ((msk[p] >> r) & 1u) continue;
-            for (int s2 = 0; s2 < 3; ++s2)
-              if (!((msk[q] >> s2) & 1u)) acc[3 * r + s2] += w * k0[24 * r + s2];
-          }
+          if (off(q, lm)) continue;
+          const double w = wp * (wm[0][q & 1] * wm[1][(q >> 1) & 1] * wm[2][q >> 2]);
+          const double *k0 = K0 + 24 * (3 * p) + 3 * q;
+#pragma unroll
+          for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              if (!(((msk[p] >> r) | (msk[q] >> c)) & 1u)) acc[3 * r + c] += w * k0[24 * r + c];
         }
       }
     }
-#pragma unroll
-    for (int q = 0; q < 9; ++q) G[(int64_t)t * 9 + q] = acc[q];
   }
+#pragma unroll
+  for (int q = 0; q < 9; ++q) sum[i][q][lane] = acc[q];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 288; e += 256) {
+    const int s = e / 9, q = e % 9;
+    if (blockIdx.x * 32 + s >= nslots) continue;
+    double v = sum[0][q][s];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) v += sum[k][q][s];
+    G[((int64_t)(blockIdx.x * 32 + s) * 64 + blockIdx.y) * 9 + q] = v;
+  }
+}
+
+// The FP32 copy of a half-stored stencil is grouped by tiles of 32 nodes:
+// coefficient hq (0..125) of node n at ((n / 32) * 126 + hq) * 32 + n % 32,
+// so the 126 x 32 values a warp reads for its 32 nodes are one contiguous
+// 16,128-byte block that one bulk L2 prefetch covers.  The FP64 form is the
+// second half of the full stencil itself, coefficient-major, hq * nn + n.
+constexpr int kH32Tile = 32;
+__host__ __device__ __forceinline__ int64_t h32_index(int hq, int64_t n) {
+  return ((n / kH32Tile) * 126 + hq) * kH32Tile + n % kH32Tile;
 }
 
 // the level-1 stencil: per (coarse node, neighbour) block, the fast-path
 // element sums, the general-path blocks of flagged elements and the
-// P^T (I - M) P term of the identity dofs
-__global__ void k_galerkin_fine(int nelx, int nely, int nelz,
-                                const double *__restrict__ E,
-                                const uint8_t *__restrict__ idm,
-                                const int *__restrict__ slot,
-                                const double *__restrict__ G,
-                                const double *__restrict__ GMi,
-                                double *__restrict__ Sc) {
+// P^T (I - M) P term of the identity dofs.  blockIdx.y = h: the centre block
+// (h = 0) and the 13 forward ones, nb = 13 + h; the operator is symmetric, so
+// the block goes, transposed, to the neighbour as well (26 - nb).  h fixes
+// the elements a block sums over and their GMi blocks, so those are uniform
+// over a CTA and come from shared memory, two at a time, for the two nodes
+// of a thread.  (Every block summed by itself, GMi read through L1, took 416
+// us at 192x96x96, and a second pass of 126 us split off the half stencil;
+// this form takes 225 us; its 570 MB of writes would take 88 us and its FP64
+// arithmetic 33 us.)  The FP32 half stencil and
+// the inverse diagonal are written on the way.
+constexpr int kGfThreads = 128, kGfNodes = 2;
+__global__ void __launch_bounds__(kGfThreads)
+    k_galerkin_fine(int nelx, int nely, int nelz, const double *__restrict__ E,
+                    const uint8_t *__restrict__ idm, const int *__restrict__ slot,
+                    const double *__restrict__ G, const double *__restrict__ GMi,
+                    double *__restrict__ Sc, float *__restrict__ H32,
+                    double *__restrict__ dinv64, float *__restrict__ dinv32) {
+  // GMi blocks of this h: (element, i) x 9, padded to 10 for 16-byte reads
+  __shared__ __align__(16) double Gs[8 * 8 * 10];
   const int fx = nelx + 1, fy = nely + 1, fz = nelz + 1;
   const int cx = (fx + 1) / 2, cy = (fy + 1) / 2, cz = (fz + 1) / 2;
   const int ncx = (nelx + 1) / 2, ncy = (nely + 1) / 2, ncz = (nelz + 1) / 2;
-  const int64_t nnc = (int64_t)cx * cy * cz;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 27 * nnc;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int nb = (int)(t / nnc);
-    const int64_t I = t - (int64_t)nb * nnc;
-    const int ix = (int)(I % cx), iy = (int)((I / cx) % cy), iz = (int)(I / ((int64_t)cx * cy));
-    const int jx = ix + nb % 3 - 1, jy = iy + (nb / 3) % 3 - 1, jz = iz + nb / 9 - 1;
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (jx >= 0 && jx < cx && jy >= 0 && jy < cy && jz >= 0 && jz < cz) {
-      bool anyflag = false;
-      for (int EK = max(iz, jz) - 1; EK <= min(iz, jz); ++EK)
-        for (int EJ = max(iy, jy) - 1; EJ <= min(iy, jy); ++EJ)
-          for (int EI = max(ix, jx) - 1; EI <= min(ix, jx); ++EI) {
-            if (EI < 0 || EJ < 0 || EK < 0 || EI >= ncx || EJ >= ncy || EK >= ncz)
-              continue;
-            const int ln = (ix - EI) + 2 * (iy - EJ) + 4 * (iz - EK);
-            const int lm = (jx - EI) + 2 * (jy - EJ) + 4 * (jz - EK);
-            const int sl = slot[((int64_t)EK * ncy + EJ) * ncx + EI];
-            if (sl >= 0) {
-              anyflag = true;
-              const double *g = G + ((int64_t)sl * 64 + ln * 8 + lm) * 9;
+  const int nnc = cx * cy * cz;
+  const int h = blockIdx.y, nb = 13 + h;
+  const int dx = nb % 3 - 1, dy = (nb / 3) % 3 - 1, dz = nb / 9 - 1;
+  // the elements holding both nodes: EI = ix - 1 + a with a in [a0, a1]
+  const int a0 = dx > 0, a1 = dx >= 0, b0 = dy > 0, b1 = dy >= 0, c0 = dz > 0, c1 = dz >= 0;
+  const int na = a1 - a0 + 1, nbb = b1 - b0 + 1, nel = na * nbb * (c1 - c0 + 1);
+  for (int t = threadIdx.x; t < nel * 72; t += kGfThreads) {
+    const int e = t / 72, i = (t / 9) % 8, q = t % 9;
+    const int a = a0 + e % na, b = b0 + (e / na) % nbb, c = c0 + e / (na * nbb);
+    const int ln = (1 - a) + 2 * (1 - b) + 4 * (1 - c);
+    const int lm = (1 - a + dx) + 2 * (1 - b + dy) + 4 * (1 - c + dz);
+    Gs[(e * 8 + i) * 10 + q] = GMi[((i * 8 + ln) * 8 + lm) * 9 + q];
+  }
+  __syncthreads();
+  int I[kGfNodes], ix[kGfNodes], iy[kGfNodes], iz[kGfNodes];
+  double acc[kGfNodes][9];
+  bool anyflag[kGfNodes];
 #pragma unroll
-              for (int q = 0; q < 9; ++q) acc[q] += g[q];
-              continue;
-            }
-            for (int i = 0; i < 8; ++i) {
-              const int ex = 2 * EI + (i & 1), ey = 2 * EJ + ((i >> 1) & 1),
-                        ez = 2 * EK + ((i >> 2) & 1);
-              const double Ee = E[((int64_t)ez * nely + ey) * nelx + ex];
-              const double *m = GMi + ((i * 8 + ln) * 8 + lm) * 9;
+  for (int u = 0; u < kGfNodes; ++u) {
+    I[u] = (blockIdx.x * kGfNodes + u) * kGfThreads + threadIdx.x;
+    const int n = min(I[u], nnc - 1);
+    ix[u] = n % cx;
+    iy[u] = (n / cx) % cy;
+    iz[u] = n / (cx * cy);
+    anyflag[u] = false;
 #pragma unroll
-              for (int q = 0; q < 9; ++q) acc[q] += Ee * __ldg(m + q);
-            }
-          }
-      if (anyflag) {
-        // P^T (I - M) P: identity dofs in the support of both N and M
-        for (int gz = max(2 * iz, 2 * jz) - 1; gz <= min(2 * iz, 2 * jz) + 1; ++gz)
-          for (int gy = max(2 * iy, 2 * jy) - 1; gy <= min(2 * iy, 2 * jy) + 1; ++gy)
-            for (int gx = max(2 * ix, 2 * jx) - 1; gx <= min(2 * ix, 2 * jx) + 1; ++gx) {
-              if (gx < 0 || gy < 0 || gz < 0 || gx >= fx || gy >= fy || gz >= fz) continue;
-              const unsigned bits = idm[((int64_t)gz * fy + gy) * fx + gx];
-              if (!bits) continue;
-              const double w = pw1(gx, ix, fx) * pw1(gy, iy, fy) * pw1(gz, iz, fz) *
-                               pw1(gx, jx, fx) * pw1(gy, jy, fy) * pw1(gz, jz, fz);
-              for (int c = 0; c < 3; ++c)
-                if ((bits >> c) & 1u) acc[4 * c] += w;
-            }
+    for (int q = 0; q < 9; ++q) acc[u][q] = 0.0;
+  }
+  for (int e = 0; e < nel; ++e) {
+    const int a = a0 + (e & (na - 1)), b = b0 + ((e >> (na - 1)) & (nbb - 1)),
+              c = c0 + (e >> (na + nbb - 2));   // na, nbb are 1 or 2
+    // slots and moduli together; a flagged element's moduli are then dropped
+    double Ee[kGfNodes][8];
+    int sl[kGfNodes];
+#pragma unroll
+    for (int u = 0; u < kGfNodes; ++u) {
+      const int EI = ix[u] - 1 + a, EJ = iy[u] - 1 + b, EK = iz[u] - 1 + c;
+      const bool in = EI >= 0 && EJ >= 0 && EK >= 0 && EI < ncx && EJ < ncy && EK < ncz;
+      const int ei = min(max(EI, 0), ncx - 1), ej = min(max(EJ, 0), ncy - 1),
+                ek = min(max(EK, 0), ncz - 1);
+      const int s0 = slot[(ek * ncy + ej) * ncx + ei];
+      sl[u] = in ? s0 : -1;
+      // unconditional loads: an element outside is clamped and zeroed below;
+      // a missing last fine element (odd counts) belongs to a flagged one
+      const int ox = 2 * ei + 1 < nelx, oy = 2 * ej + 1 < nely ? nelx : 0,
+                oz = 2 * ek + 1 < nelz ? nelx * nely : 0;
+      const double *row = E + ((2 * ek * nely + 2 * ej) * nelx + 2 * ei);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        Ee[u][i] = row[((i & 1) ? ox : 0) + ((i & 2) ? oy : 0) + ((i & 4) ? oz : 0)];
+      if (!in) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Ee[u][i] = 0.0;
       }
     }
 #pragma unroll
-    for (int q = 0; q < 9; ++q) Sc[(int64_t)(nb * 9 + q) * nnc + I] = acc[q];
+    for (int u = 0; u < kGfNodes; ++u)
+      if (sl[u] >= 0) {   // the general path's block instead
+        anyflag[u] = true;
+        const int ln = (1 - a) + 2 * (1 - b) + 4 * (1 - c);
+        const int lm = (1 - a + dx) + 2 * (1 - b + dy) + 4 * (1 - c + dz);
+        const double *g = G + ((int64_t)sl[u] * 64 + ln * 8 + lm) * 9;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc[u][q] += g[q];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Ee[u][i] = 0.0;
+      }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const double2 *m2 = reinterpret_cast<const double2 *>(Gs + (e * 8 + i) * 10);
+      const double2 p0 = m2[0], p1 = m2[1], p2 = m2[2], p3 = m2[3];
+      const double m[9] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y,
+                           Gs[(e * 8 + i) * 10 + 8]};
+#pragma unroll
+      for (int u = 0; u < kGfNodes; ++u)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc[u][q] = fma(Ee[u][i], m[q], acc[u][q]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kGfNodes; ++u) {
+    if (I[u] >= nnc) continue;
+    const int jx = ix[u] + dx, jy = iy[u] + dy, jz = iz[u] + dz;
+    const bool inside = jx >= 0 && jx < cx && jy >= 0 && jy < cy && jz >= 0 && jz < cz;
+    if (inside && anyflag[u]) {
+      // P^T (I - M) P: identity dofs in the support of both N and M
+      for (int gz = max(2 * iz[u], 2 * jz) - 1; gz <= min(2 * iz[u], 2 * jz) + 1; ++gz)
+        for (int gy = max(2 * iy[u], 2 * jy) - 1; gy <= min(2 * iy[u], 2 * jy) + 1; ++gy)
+          for (int gx = max(2 * ix[u], 2 * jx) - 1; gx <= min(2 * ix[u], 2 * jx) + 1; ++gx) {
+            if (gx < 0 || gy < 0 || gz < 0 || gx >= fx || gy >= fy || gz >= fz) continue;
+            const unsigned bits = idm[((int64_t)gz * fy + gy) * fx + gx];
+            if (!bits) continue;
+            const double w = pw1(gx, ix[u], fx) * pw1(gy, iy[u], fy) * pw1(gz, iz[u], fz) *
+                             pw1(gx, jx, fx) * pw1(gy, jy, fy) * pw1(gz, jz, fz);
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              if ((bits >> c) & 1u) acc[u][4 * c] += w;
+          }
+    }
+    const int J = I[u] + (dz * cy + dy) * cx + dx;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const double v = inside ? acc[u][q] : 0.0;
+      Sc[(int64_t)(nb * 9 + q) * nnc + I[u]] = v;
+      if (h > 0 && inside)
+        Sc[(int64_t)((26 - nb) * 9 + 3 * (q % 3) + q / 3) * nnc + J] = v;
+      if (H32) H32[h32_index(h * 9 + q, I[u])] = static_cast<float>(v);
+    }
+    // the backward block of a node without that neighbour
+    const int kx = ix[u] - dx, ky = iy[u] - dy, kz = iz[u] - dz;
+    if (!(kx >= 0 && kx < cx && ky >= 0 && ky < cy && kz >= 0 && kz < cz)) {
+#pragma unroll
+      for (int q = 0; q < 9; ++q) Sc[(int64_t)((26 - nb) * 9 + q) * nnc + I[u]] = 0.0;
+    }
+    if (h == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        dinv64[3 * (int64_t)I[u] + c] = 1.0 / acc[u][4 * c];
+        dinv32[3 * (int64_t)I[u] + c] = static_cast<float>(1.0 / acc[u][4 * c]);
+      }
+    }
   }
 }
 
@@ -264,11 +397,11 @@ __global__ void k_galerkin_dim(int nx, int ny, int nz, const double *__restrict_
 // shared memory in a fixed order.  Lanes span consecutive nodes, so each
 // coefficient load is coalesced.
 constexpr int kStencilRows = 9;
-template <typename T, bool RESID>
+template <typename T, int OUT>
 __global__ void __launch_bounds__(32 * kStencilRows)
     k_apply_stencil(int nx, int ny, int nz, const T *__restrict__ S,
                     const T *__restrict__ u, const T *__restrict__ b,
-                    T *__restrict__ y) {
+                    const T *__restrict__ dinv, T *__restrict__ y) {
   __shared__ T part[kStencilRows][3][32];
   const int64_t nn = (int64_t)nx * ny * nz;
   const int lane = threadIdx.x, g = threadIdx.y;
@@ -302,22 +435,14 @@ __global__ void __launch_bounds__(32 * kStencilRows)
       T a = 0;
 #pragma unroll
       for (int r = 0; r < kStencilRows; ++r) a += part[r][g][lane];
-      if (RESID) a = b[3 * n + g] - a;
+      if (OUT == OUT_RESID) a = b[3 * n + g] - a;
+      if (OUT == OUT_SCALE) a *= dinv[3 * n + g];
       y[3 * n + g] = a;
     }
     __syncthreads();
   }
 }
 
-// The FP32 copy of a half-stored stencil is grouped by tiles of 32 nodes:
-// coefficient hq (0..125) of node n at ((n / 32) * 126 + hq) * 32 + n % 32,
-// so the 126 x 32 values a warp reads for its 32 nodes are one contiguous
-// 16,128-byte block that one bulk L2 prefetch covers.  The FP64 copy stays
-// coefficient-major, hq * nn + n.
-constexpr int kH32Tile = 32;
-__host__ __device__ __forceinline__ int64_t h32_index(int hq, int64_t n) {
-  return ((n / kH32Tile) * 126 + hq) * kH32Tile + n % kH32Tile;
-}
 template <typename T>
 __device__ __forceinline__ const T *hcoef(const T *H, int hq, int64_t n, int64_t nn);
 template <>
@@ -337,22 +462,20 @@ __device__ __forceinline__ void prefetch_h32_tile(const float *H, int64_t n) {
                : "memory");
 }
 
-// Symmetric half of a Galerkin stencil: A(n, n+d) = A(n+d, n)^T, so only
-// the centre block and the 13 forward offsets (nb = 13..26) are stored,
-// H[(h*9 + 3r + s) * nn + n] with h = nb - 13.  The apply reads the forward
+// Symmetric half of a Galerkin stencil: A(n, n+d) = A(n+d, n)^T, so the
+// apply needs only the centre block and the 13 forward offsets (nb =
+// 13..26), H[(h*9 + 3r + s) * nn + n] with h = nb - 13: in FP64 the second
+// half of the stencil in place, in FP32 a copy.  The apply reads the forward
 // blocks of node n and, transposed, the forward blocks that its 13 backward
 // neighbours store for it; those were read moments earlier by the
 // neighbouring threads, so the second read hits L2 and DRAM traffic is the
 // half-size array.
-__global__ void k_stencil_to_half(int64_t nn, const double *__restrict__ S,
-                                  double *__restrict__ H64,
+__global__ void k_stencil_to_half(int64_t nn, const double *__restrict__ H64,
                                   float *__restrict__ H32) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 126 * nn;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const double v = S[117 * nn + t];   // (13*9 + q) * nn + n
-    H64[t] = v;
     const int64_t hq = t / nn, n = t - hq * nn;
-    H32[h32_index((int)hq, n)] = static_cast<float>(v);
+    H32[h32_index((int)hq, n)] = static_cast<float>(H64[t]);
   }
 }
 
@@ -498,52 +621,173 @@ __global__ void k_stencil_diag(int64_t nn, const double *__restrict__ S,
   }
 }
 
+// The transfers are separable, P = Px (x) Py (x) Pz, and both kernels give a
+// thread one coarse index along x for one coarse (restriction) or fine
+// (prolongation) y and z: consecutive lanes are consecutive coarse nodes, each
+// value is loaded once per (y, z) pair that needs it, and the x direction takes
+// the neighbouring lane's value (the lane at a warp's edge loads it).  One
+// thread per output node with all of its 27 or 8 taps took, at 192x96x96 in
+// FP32, 17 us for the restriction and 29 us for the prolongation (8 and 10 us
+// on level 1); these take 10 and 17 us (6 and 6 us); 8 columns of 128x64x64,
+// 37 and 44 us before, 19 and 35 us now.  A copy of the bytes takes 4 and 7
+// us; both are bound by their instructions.
+
+// weights of the three fine indices 2 c - 1, 2 c, 2 c + 1 around coarse c
+template <typename T>
+__device__ __forceinline__ void tap_weights(int c, int N, T (&w)[3]) {
+  const int f = 2 * c;
+  w[0] = f - 1 >= 0 ? T(0.5) : T(0);
+  w[1] = T(1);
+  w[2] = f + 1 < N ? (f + 2 < N ? T(0.5) : T(1)) : T(0);
+}
+
 // b_c = P^T r_f for nb columns (fine stride 3 nnf, coarse stride 3 nnc);
-// COMP: b_c component by component, with the first Chebyshev direction
+// COMP: b_c component by component, with the first Chebyshev direction.
+// blockIdx.z = column; a thread per coarse node
 template <typename T, bool COMP>
-__global__ void k_restrict(int fx, int fy, int fz, int cx, int cy, int cz,
-                           const T *__restrict__ rf, T *__restrict__ bc,
-                           const CompLevel<T> comp, int nb) {
-  const int64_t nnc = (int64_t)cx * cy * cz, nnf = (int64_t)fx * fy * fz;
-  for (int64_t I = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; I < nnc;
-       I += (int64_t)gridDim.x * blockDim.x) {
-    const int ix = I % cx, iy = (I / cx) % cy, iz = I / ((int64_t)cx * cy);
-    for (int col = 0; col < nb; ++col) {
-      T s[3];
-      restrict_node(fx, fy, fz, ix, iy, iz, rf + col * 3 * nnf, s);
-      T *o = bc + col * 3 * nnc;
+__global__ void __launch_bounds__(128)
+    k_restrict(int fx, int fy, int fz, int cx, int cy, int cz, const T *__restrict__ rf,
+               T *__restrict__ bc, const CompLevel<T> comp) {
+  const int lane = threadIdx.x & 31;
+  const int nnc = cx * cy * cz, t = (int)blockIdx.x * 128 + threadIdx.x;
+  const int I = min(t, nnc - 1);
+  const int ix = I % cx, iy = (I / cx) % cy, iz = I / (cx * cy);
+  const int col = blockIdx.z;
+  rf += col * 3 * ((int64_t)fx * fy * fz);
+  T wx[3], wy[3], wz[3];
+  tap_weights(ix, fx, wx);
+  tap_weights(iy, fy, wy);
+  tap_weights(iz, fz, wz);
+  const bool first = lane == 0 && ix > 0;   // loads its own left neighbour
+  T s[3] = {T(0), T(0), T(0)};
+  const int dl = ix > 0 ? -3 : 0, d1 = 2 * ix + 1 < fx ? 3 : 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        if (COMP) {
-          o[c * nnc + I] = s[c];
-          comp.d0[(3 * col + c) * nnc + I] = comp.inv_theta * (comp.dinv[3 * I + c] * s[c]);
-        } else {
-          o[3 * I + c] = s[c];
-        }
+  for (int c = 0; c < 3; ++c) {
+    const int z = min(max(2 * iz + c - 1, 0), fz - 1);
+    T a0[3][3], a1[3][3], am[3][3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int y = min(max(2 * iy + b - 1, 0), fy - 1);
+      const T *p = rf + 3 * ((z * fy + y) * fx + 2 * ix);   // 32-bit: 3 nn < 2^31
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        a0[b][q] = p[q];
+        a1[b][q] = p[d1 + q];
+        am[b][q] = first ? p[dl + q] : T(0);
       }
+    }
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const T wyz = wy[b] * wz[c];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        T left = __shfl_up_sync(0xffffffffu, a1[b][q], 1);
+        if (lane == 0 || ix == 0) left = am[b][q];
+        s[q] += wyz * (wx[0] * left + a0[b][q] + wx[2] * a1[b][q]);
+      }
+    }
+  }
+  if (t >= nnc) return;
+  T *o = bc + col * 3 * (int64_t)nnc;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (COMP) {
+      o[q * (int64_t)nnc + I] = s[q];
+      comp.d0[(3 * col + q) * (int64_t)nnc + I] = comp.inv_theta * (comp.dinv[3 * I + q] * s[q]);
+    } else {
+      o[3 * I + q] = s[q];
     }
   }
 }
 
-// x_f += P x_c for nb columns; COMP: x_c component by component
+// x_f += P x_c for nb columns; COMP: x_c component by component.
+// blockIdx.z = column; a thread per (coarse ix, fine gy, gz), writing the fine
+// nodes 2 ix and 2 ix + 1
 template <typename T, bool COMP>
-__global__ void k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz,
-                              const T *__restrict__ xc, T *__restrict__ xf,
-                              int nb) {
-  const int64_t nnf = (int64_t)fx * fy * fz, nnc = (int64_t)cx * cy * cz;
-  for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nnf;
-       f += (int64_t)gridDim.x * blockDim.x) {
-    const int gx = f % fx, gy = (f / fx) % fy, gz = f / ((int64_t)fx * fy);
-    for (int col = 0; col < nb; ++col) {
-      T s[3];
-      prolong_node(fx, fy, fz, cx, cy, cz, gx, gy, gz, xc + col * 3 * nnc, COMP ? 1 : 3,
-                   COMP ? nnc : 1, s);
-      T *o = xf + col * 3 * nnf;
-      o[3 * f] += s[0];
-      o[3 * f + 1] += s[1];
-      o[3 * f + 2] += s[2];
+__global__ void __launch_bounds__(128)
+    k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz, const T *__restrict__ xc,
+                  T *__restrict__ xf) {
+  const int lane = threadIdx.x & 31;
+  const int total = cx * fy * fz, t = (int)blockIdx.x * 128 + threadIdx.x;
+  const int i = min(t, total - 1);
+  const int ix = i % cx, gy = (i / cx) % fy, gz = i / (cx * fy);
+  const int nnc = cx * cy * cz;
+  xc += (int64_t)blockIdx.z * 3 * nnc;
+  xf += (int64_t)blockIdx.z * 3 * ((int64_t)fx * fy * fz);
+  // within a column 32-bit offsets reach (3 nn < 2^31): the kernel is bound
+  // by its instructions
+  const int sn = COMP ? 1 : 3, sc = COMP ? nnc : 1;
+  // one or two coarse rows in y and in z
+  const bool ty = (gy & 1) && gy + 1 < fy, tz = (gz & 1) && gz + 1 < fz;
+  const T wyz = (ty ? T(0.5) : T(1)) * (tz ? T(0.5) : T(1));
+  const int o00 = (((gz >> 1) * cy + (gy >> 1)) * cx + ix) * sn;
+  const int dy = cx * sn, dz = cx * cy * sn, dr = ix + 1 < cx ? sn : 0;
+  const bool last = lane == 31;   // loads its own right neighbour
+  T v[3] = {T(0), T(0), T(0)}, r[3] = {T(0), T(0), T(0)};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (((k & 1) && !ty) || ((k >> 1) && !tz)) continue;
+    const T *p = xc + (o00 + ((k & 1) ? dy : 0) + ((k >> 1) ? dz : 0));
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      v[q] += p[q * sc];
+      if (last) r[q] += p[dr + q * sc];
     }
   }
+  // the warp's 32 x 6 corrections through shared memory, so that the fine
+  // vector is read and written by consecutive lanes (each lane its own 24
+  // bytes took 20 us of partial-sector writes)
+  __shared__ T vals[4][192];
+  __shared__ int base[4][32];   // first dof of the lane's pair
+  const int wp = threadIdx.x >> 5;
+  const bool odd = 2 * ix + 1 < fx, tx = 2 * ix + 2 < fx;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    v[q] *= wyz;
+    T right = __shfl_down_sync(0xffffffffu, v[q], 1);
+    if (last) right = r[q] * wyz;
+    vals[wp][6 * lane + q] = v[q];
+    vals[wp][6 * lane + 3 + q] = tx ? T(0.5) * v[q] + T(0.5) * right : v[q];
+  }
+  // nodes of the pair: 2, 1 (odd last node missing) or 0 (past the end), as
+  // one ballot each
+  base[wp][lane] = 3 * ((gz * fy + gy) * fx + 2 * ix);
+  const unsigned has0 = __ballot_sync(0xffffffffu, t < total);
+  const unsigned has1 = __ballot_sync(0xffffffffu, t < total && odd);
+  __syncwarp();
+  T f[6];
+  int at[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const unsigned e = lane + 32 * k, o = e / 6u, c = e - 6 * o;
+    const bool in = ((c < 3 ? has0 : has1) >> o) & 1u;
+    at[k] = in ? base[wp][o] + (int)c : -1;
+    f[k] = in ? xf[at[k]] : T(0);
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    if (at[k] >= 0) xf[at[k]] = f[k] + vals[wp][lane + 32 * k];
+}
+
+// one row of x = Ainv b by one warp: four independent partial sums so the
+// loads of consecutive chunks overlap; result valid in every lane
+template <typename T>
+__device__ __forceinline__ double gemv_row(const double *__restrict__ a,
+                                           const T *__restrict__ b, int64_t n,
+                                           int lane) {
+  double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+  int64_t k = lane;
+  for (; k + 96 < n; k += 128) {
+    s0 += a[k] * static_cast<double>(b[k]);
+    s1 += a[k + 32] * static_cast<double>(b[k + 32]);
+    s2 += a[k + 64] * static_cast<double>(b[k + 64]);
+    s3 += a[k + 96] * static_cast<double>(b[k + 96]);
+  }
+  for (; k < n; k += 32) s0 += a[k] * static_cast<double>(b[k]);
+  double s = (s0 + s1) + (s2 + s3);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
 }
 
 // x = Ainv b, one warp per row, FP64 accumulation
@@ -605,23 +849,24 @@ __global__ void k_cheb_step(int64_t n, const T *__restrict__ dinv,
 
 template <typename T>
 void launch_apply_stencil(const Level &v, const T *S, const T *u, const T *b,
-                          T *y, cudaStream_t s) {
+                          T *y, cudaStream_t s, const T *scale) {
   count_launch();
   const int g = grid_for(v.nn, 32);
   const dim3 blk(32, kStencilRows);
-  if (b)
-    k_apply_stencil<T, true><<<g, blk, 0, s>>>(v.dims[0], v.dims[1], v.dims[2],
-                                               S, u, b, y);
+  const int nx = v.dims[0], ny = v.dims[1], nz = v.dims[2];
+  if (scale)
+    k_apply_stencil<T, OUT_SCALE><<<g, blk, 0, s>>>(nx, ny, nz, S, u, nullptr, scale, y);
+  else if (b)
+    k_apply_stencil<T, OUT_RESID><<<g, blk, 0, s>>>(nx, ny, nz, S, u, b, nullptr, y);
   else
-    k_apply_stencil<T, false><<<g, blk, 0, s>>>(v.dims[0], v.dims[1], v.dims[2],
-                                                S, u, b, y);
+    k_apply_stencil<T, OUT_Y><<<g, blk, 0, s>>>(nx, ny, nz, S, u, nullptr, nullptr, y);
 }
 template void launch_apply_stencil<double>(const Level &, const double *,
                                            const double *, const double *,
-                                           double *, cudaStream_t);
+                                           double *, cudaStream_t, const double *);
 template void launch_apply_stencil<float>(const Level &, const float *,
                                           const float *, const float *, float *,
-                                          cudaStream_t);
+                                          cudaStream_t, const float *);
 
 template <typename T, bool RESID, int NB>
 void sym_launch(const Level &v, const T *H, const T *u, const T *b, T *y,
@@ -673,6 +918,8 @@ void launch_apply_sym_fused(const Level &v, const T *H, int in, int out,
     k_apply_stencil_sym1<T, IN_U, OUT_POST1><<<g, 128, 0, s>>>(nx, ny, nz, H, a);
   else if (out == OUT_RESID)
     k_apply_stencil_sym1<T, IN_U, OUT_RESID><<<g, 128, 0, s>>>(nx, ny, nz, H, a);
+  else if (out == OUT_SCALE)
+    k_apply_stencil_sym1<T, IN_U, OUT_SCALE><<<g, 128, 0, s>>>(nx, ny, nz, H, a);
   else
     k_apply_stencil_sym1<T, IN_U, OUT_Y><<<g, 128, 0, s>>>(nx, ny, nz, H, a);
 }
@@ -696,10 +943,9 @@ template void launch_apply_stencil_sym<float>(const Level &, const float *,
                                               const float *, const float *,
                                               float *, cudaStream_t, int);
 
-void launch_stencil_to_half(int64_t nn, const double *S, double *H64,
-                            float *H32, cudaStream_t s) {
+void launch_stencil_to_half(int64_t nn, const double *H64, float *H32, cudaStream_t s) {
   count_launch();
-  k_stencil_to_half<<<grid_for(126 * nn, 256), 256, 0, s>>>(nn, S, H64, H32);
+  k_stencil_to_half<<<grid_for(126 * nn, 256), 256, 0, s>>>(nn, H64, H32);
 }
 
 int launch_galerkin_fine(Ctx &c, double *Sc, cudaStream_t s) {
@@ -725,15 +971,17 @@ int launch_galerkin_fine(Ctx &c, double *Sc, cudaStream_t s) {
   }
   if (nslots) {
     count_launch();
-    k_galerkin_general<<<grid_for(64 * (int64_t)nslots, 128, 1 << 20), 128, 0, s>>>(
-        c.nel[0], c.nel[1], c.nel[2], (int)nslots, c.E64, c.idm, c.gk_elem, c.K0lex,
-        c.gk_G);
+    k_galerkin_general<<<dim3((nslots + 31) / 32, 64), 256, 0, s>>>(
+        c.nel[0], c.nel[1], c.nel[2], (int)nslots, c.E64, c.idm, c.gk_elem, c.K0lex, c.GMi, c.gk_G);
   }
   count_launch();
-  k_galerkin_fine<<<grid_for(27 * c.lev[1].nn, 128, 1 << 20), 128, 0, s>>>(
-      c.nel[0], c.nel[1], c.nel[2], c.E64, c.idm, c.gk_slot, c.gk_G, c.GMi, Sc);
-  // the tensor-core form of the FP32 level-1 operator (kernels_l1tc.cu)
-  return l1tc_prepare(c, Sc, (int)nslots, s);
+  Level &v = c.lev[1];
+  const dim3 grid((unsigned)((v.nn + kGfThreads * kGfNodes - 1) / (kGfThreads * kGfNodes)), 14);
+  k_galerkin_fine<<<grid, kGfThreads, 0, s>>>(c.nel[0], c.nel[1], c.nel[2], c.E64, c.idm,
+                                              c.gk_slot, c.gk_G, c.GMi, Sc, v.H32, v.dinv64,
+                                              v.dinv32);
+  c.gk_nslots = (int)nslots;
+  return TPO_OK;
 }
 
 void launch_galerkin_dims(const Level &fine, const double *Sf, double *Sc,
@@ -766,15 +1014,13 @@ template <typename T>
 void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *bc,
                      const CompLevel<T> *comp, cudaStream_t s, int nb) {
   count_launch();
-  const int g = grid_for(coarse.nn, 128);
+  const int *f = fine.dims, *c = coarse.dims;
+  const dim3 g((unsigned)((coarse.nn + 127) / 128), 1, nb);
   if (comp)
-    k_restrict<T, true><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
-                                          coarse.dims[0], coarse.dims[1], coarse.dims[2], rf, bc,
-                                          *comp, nb);
+    k_restrict<T, true><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], rf, bc, *comp);
   else
-    k_restrict<T, false><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
-                                           coarse.dims[0], coarse.dims[1], coarse.dims[2], rf, bc,
-                                           CompLevel<T>{}, nb);
+    k_restrict<T, false><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], rf, bc,
+                                           CompLevel<T>{});
 }
 template void launch_restrict<double>(const Level &, const Level &, const double *, double *,
                                       const CompLevel<double> *, cudaStream_t, int);
@@ -785,15 +1031,12 @@ template <typename T>
 void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc, T *xf, bool comp,
                         cudaStream_t s, int nb) {
   count_launch();
-  const int g = grid_for(fine.nn, 128);
+  const int *f = fine.dims, *c = coarse.dims;
+  const dim3 g((unsigned)(((int64_t)c[0] * f[1] * f[2] + 127) / 128), 1, nb);
   if (comp)
-    k_prolong_add<T, true><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
-                                             coarse.dims[0], coarse.dims[1], coarse.dims[2], xc,
-                                             xf, nb);
+    k_prolong_add<T, true><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
   else
-    k_prolong_add<T, false><<<g, 128, 0, s>>>(fine.dims[0], fine.dims[1], fine.dims[2],
-                                              coarse.dims[0], coarse.dims[1], coarse.dims[2], xc,
-                                              xf, nb);
+    k_prolong_add<T, false><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
 }
 template void launch_prolong_add<double>(const Level &, const Level &, const double *, double *,
                                          bool, cudaStream_t, int);

@@ -243,22 +243,6 @@ __global__ void k_power_start(int64_t n, T *a) {
     a[i] = static_cast<T>(start_value((uint64_t)i));
 }
 
-// w *= dinv and ||w||^2, accumulated in FP64 for either storage type
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads)
-    k_scale_diag_dot(int64_t n, T *__restrict__ w, const T *__restrict__ dinv,
-                     double *part, unsigned int *ticket, double *out,
-                     double *shift_to) {
-  double s = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const T wi = w[i] * dinv[i];
-    w[i] = wi;
-    s += static_cast<double>(wi) * static_cast<double>(wi);
-  }
-  finish_reduction(s, part, ticket, out, shift_to);
-}
-
 // b = float(a / sqrt(*nrm2)) per column (a zero column stays zero)
 __global__ void k_to_f32_scaled(int64_t n, const double *a, const double *nrm2,
                                 float *b) {
@@ -374,21 +358,6 @@ void launch_power_start(int64_t n, T *a, cudaStream_t s) {
 }
 template void launch_power_start<double>(int64_t, double *, cudaStream_t);
 template void launch_power_start<float>(int64_t, float *, cudaStream_t);
-
-template <typename T>
-void launch_scale_diag_dot(const Ctx &c, int64_t n, T *w, const T *dinv, double *out,
-                           double *shift_to, cudaStream_t s, double *part,
-                           unsigned int *ticket) {
-  count_launch();
-  k_scale_diag_dot<T><<<red_grid(1), kRedThreads, 0, s>>>(
-      n, w, dinv, part ? part : c.part, ticket ? ticket : c.ticket, out, shift_to);
-}
-template void launch_scale_diag_dot<double>(const Ctx &, int64_t, double *, const double *,
-                                            double *, double *, cudaStream_t, double *,
-                                            unsigned int *);
-template void launch_scale_diag_dot<float>(const Ctx &, int64_t, float *, const float *,
-                                           double *, double *, cudaStream_t, double *,
-                                           unsigned int *);
 
 void launch_to_f32_scaled(int64_t n, const double *a, const double *scal,
                           float *b, cudaStream_t s, int nb) {

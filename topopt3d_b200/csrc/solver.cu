@@ -566,14 +566,39 @@ void invalidate_graphs(Ctx &c) {
   c.graph64_nb = c.graph32_nb = 0;
 }
 
+// w = D^-1 A_l a, in the operator kernels' epilogue
+template <typename T>
+void level_scaled_apply(Ctx &c, int l, const T *a, T *w, cudaStream_t s) {
+  Level &v = c.lev[l];
+  LV<T> wv = lv(v, (T *)nullptr);
+  ApplyArgs<T> ar{};
+  ar.u = a;
+  ar.dinv = wv.dinv;
+  ar.y = w;
+  if (l == 0) {
+    launch_apply_fused<T>(c, fineE(c, (T *)nullptr), IN_U, OUT_SCALE, ar, s);
+  } else if (l < c.ps) {
+    if constexpr (std::is_same<T, float>::value) {
+      if (l == 1 && l1_tensor(c)) {
+        launch_l1tc(c, IN_U, OUT_SCALE, ar, s);
+        return;
+      }
+    }
+    launch_apply_sym_fused<T>(v, halfS(v, (T *)nullptr), IN_U, OUT_SCALE, ar, s);
+  } else {
+    launch_apply_stencil<T>(v, wv.S, a, nullptr, w, s, wv.dinv);
+  }
+}
+
 // power iteration for lambda_max(D^-1 A_l) on stream s, no host sync.  The
 // start vector is the splitmix64 sequence the oracle shares.  The iterates
 // v_{k+1} = D^-1 A v_k are not normalised (lambda_max(D^-1 A) is a small
-// number, so 15 steps stay far inside the FP64 range): each step is the
-// apply and one fused pass for the diagonal scaling and the squared norm,
-// which leaves ||v_k||^2 in scal[SC_POWER + l] and ||v_{k-1}||^2 in
-// scal[SC_POWER_PREV + l].  lambda = ||v_k|| / ||v_{k-1}|| is then the
+// number, so 15 steps stay far inside the FP64 range), so a step is one
+// launch, and only the last two squared norms are formed: scal[SC_POWER_PREV
+// + l] and scal[SC_POWER + l].  lambda = ||v_k|| / ||v_{k-1}|| is then the
 // estimate ||D^-1 A a|| of the normalised iteration, a = v_{k-1}/||v_{k-1}||.
+// (A separate scaling and norm pass per step took 12 us of the 45 us a step
+// on the fine level of 192x96x96, 6 of 18 us on the small levels.)
 template <typename T>
 void power_iteration_t(Ctx &c, int l, int its, cudaStream_t s, double *part,
                        unsigned int *ticket) {
@@ -581,14 +606,14 @@ void power_iteration_t(Ctx &c, int l, int its, cudaStream_t s, double *part,
   const int64_t n = 3 * v.nn;
   LV<T> wv = lv(v, (T *)nullptr);
   T *a = wv.d, *w = wv.a;
-  double *nrm = c.scal + SC_POWER + l, *prev = c.scal + SC_POWER_PREV + l;
   launch_power_start<T>(n, a, s);
-  launch_dot<T>(c, n, a, a, nrm, nullptr, s, 1, part, ticket);
   for (int k = 0; k < its; ++k) {
-    level_apply<T>(c, l, a, nullptr, w, s);
-    launch_scale_diag_dot<T>(c, n, w, wv.dinv, nrm, prev, s, part, ticket);
+    if (k == its - 1)
+      launch_dot<T>(c, n, a, a, c.scal + SC_POWER_PREV + l, nullptr, s, 1, part, ticket);
+    level_scaled_apply<T>(c, l, a, w, s);
     std::swap(a, w);
   }
+  launch_dot<T>(c, n, a, a, c.scal + SC_POWER + l, nullptr, s, 1, part, ticket);
 }
 
 // fp32: the hierarchy is set up for the mixed form, whose smoothers run in
@@ -636,6 +661,9 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
     const int i = l % kAuxStreams;
     CK(cudaEventRecord(c.lev_ev[l], s));
     CK(cudaStreamWaitEvent(c.aux_stream[i], c.lev_ev[l], 0));
+    // the tensor-core form of the FP32 level-1 operator (kernels_l1tc.cu)
+    if (l == 1)
+      if (int rc = l1tc_prepare(c, c.lev[1].S64, c.gk_nslots, c.aux_stream[i])) return rc;
     power_iteration(c, l, o.power_its, c.aux_stream[i],
                     c.part + kAuxPart + i * kRedBlocks, c.ticket + kMaxBatch + i,
                     o.precision == TPO_PREC_MIXED);
@@ -662,11 +690,11 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
     } else {
       launch_galerkin_dims(c.lev[l], c.lev[l].S64, c.lev[l + 1].S64, c.gd_tmp, s);
     }
-    launch_stencil_diag(c.lev[l + 1], c.lev[l + 1].S64, c.lev[l + 1].dinv64,
-                        c.lev[l + 1].dinv32, s);
-    if (l + 1 < c.ps) {
-      launch_stencil_to_half(c.lev[l + 1].nn, c.lev[l + 1].S64, c.lev[l + 1].H64,
-                             c.lev[l + 1].H32, s);
+    if (l > 0) {   // level 1 comes with both
+      launch_stencil_diag(c.lev[l + 1], c.lev[l + 1].S64, c.lev[l + 1].dinv64,
+                          c.lev[l + 1].dinv32, s);
+      if (l + 1 < c.ps)
+        launch_stencil_to_half(c.lev[l + 1].nn, c.lev[l + 1].H64, c.lev[l + 1].H32, s);
     }
     if (l + 1 >= c.ps && l + 1 < c.L - 1)
       launch_coarse_slabs(c.lev[l + 1], coarse_ctas(c.device), c.lev[l + 1].S64,
@@ -686,6 +714,8 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
   c.nc = nc;
   launch_coarse_inverse(cl, Sc, c.inv, c.Ainv, c.Adense, c.dev_info, s);
   CK(cudaGetLastError());
+  // the side streams: Chebyshev bounds, the level-1 correction rows
+  join();
   int info_h = 0, l1_fault_h = 0;
   unsigned int l1_rows_h = 0;
   CK(cudaMemcpyAsync(&info_h, c.dev_info, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -693,25 +723,20 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
     CK(cudaMemcpyAsync(&l1_fault_h, c.l1_fault, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&l1_rows_h, c.l1_count, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
   }
+  CK(cudaMemcpyAsync(c.scal_h + SC_POWER, c.scal + SC_POWER,
+                     sizeof(double) * (SC_POWER_PREV + kMaxLevels - SC_POWER),
+                     cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   c.l1_nrows = (int)std::min<size_t>(l1_rows_h, c.l1_cap);
   if (l1_fault_h != 0) {
     c.err = "level-1 correction rows exceed their capacity";
-    join();
     return TPO_E_CUDA;
   }
   if (info_h != 0) {
     c.err = "coarsest operator is not positive definite (pivot " +
             std::to_string(info_h - 1) + ")";
-    join();
     return TPO_E_BREAKDOWN;
   }
-  // Chebyshev bounds from the side stream
-  join();
-  CK(cudaMemcpyAsync(c.scal_h + SC_POWER, c.scal + SC_POWER,
-                     sizeof(double) * (SC_POWER_PREV + kMaxLevels - SC_POWER),
-                     cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
   for (int l = 0; l + 1 < c.L; ++l) c.lev[l].lam = power_lambda(c, l);
   c.setup_opts = o;
   c.assembled = true;

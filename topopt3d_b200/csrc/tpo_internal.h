@@ -77,7 +77,8 @@ struct Level {
   double *A64 = nullptr;
   float *A32 = nullptr;
   // symmetric half (centre + 13 forward blocks) for the levels between the
-  // finest and the persistent kernel: H[(h*9 + 3r + s) * nn + n]
+  // finest and the persistent kernel: H64 = the second half of S64, H[(h*9 +
+  // 3r + s) * nn + n]; H32 a copy by tiles (kernels_mg.cu)
   double *H64 = nullptr;
   float *H32 = nullptr;
   double *dinv64 = nullptr;
@@ -183,6 +184,7 @@ struct Ctx {
   unsigned int *gk_count = nullptr;
   double *gk_G = nullptr;
   size_t gk_cap = 0;
+  int gk_nslots = 0;   // general-path elements of the last assembly
   // level 1 in FP32 on the tensor cores (kernels_l1tc.cu): the form
   // requested (0 automatic, 1 always the stored stencil), whether the
   // context qualifies (even element counts, level 1 above the persistent
@@ -318,7 +320,7 @@ void launch_apply_fine(const Ctx &c, const T *E, const T *u, const T *b, T *y,
 // fused fine-level variants: how the input is formed and what the epilogue
 // writes (sym_out_v, fused_out.cuh)
 enum { IN_U = 0, IN_CHEB = 1 };
-enum { OUT_Y = 0, OUT_RESID = 1, OUT_CHEB2 = 2, OUT_POST0 = 3, OUT_POST1 = 4 };
+enum { OUT_Y = 0, OUT_RESID = 1, OUT_CHEB2 = 2, OUT_POST0 = 3, OUT_POST1 = 4, OUT_SCALE = 5 };
 
 // u, b, y, y2 are per column (stride ld); dinv is shared by the columns
 template <typename T>
@@ -339,9 +341,10 @@ void launch_fine_stencil(const Ctx &c, double *S, cudaStream_t s);
 void launch_identity_mask(const Ctx &c, cudaStream_t s);
 
 // stencil levels
+// scale: y = D^-1 A u (b unused)
 template <typename T>
 void launch_apply_stencil(const Level &v, const T *S, const T *u, const T *b,
-                          T *y, cudaStream_t s);
+                          T *y, cudaStream_t s, const T *scale = nullptr);
 template <typename T>
 void launch_apply_stencil_sym(const Level &v, const T *H, const T *u,
                               const T *b, T *y, cudaStream_t s, int nb = 1);
@@ -350,8 +353,7 @@ void launch_apply_stencil_sym(const Level &v, const T *H, const T *u,
 template <typename T>
 void launch_apply_sym_fused(const Level &v, const T *H, int in, int out,
                             const ApplyArgs<T> &a, cudaStream_t s);
-void launch_stencil_to_half(int64_t nn, const double *S, double *H64,
-                            float *H32, cudaStream_t s);
+void launch_stencil_to_half(int64_t nn, const double *H64, float *H32, cudaStream_t s);
 // level 1 on the tensor cores (kernels_l1tc.cu)
 // true when the FP32 level-1 operator runs on the tensor-core kernel
 inline bool l1_tensor(const Ctx &c) { return c.l1tc_ok && c.l1_form == 0; }
@@ -369,7 +371,8 @@ void l1tc_grid(const Level &v, int *tx, int *ty, int *zchunk, int *nz);
 void launch_galerkin_dims(const Level &fine, const double *Sf, double *Sc,
                           double *tmp, cudaStream_t s);
 size_t galerkin_dims_scratch(const Level &fine);
-// level 1 = P^T A_0 P from the element moduli (no fine stencil); syncs
+// level 1 = P^T A_0 P from the element moduli (no fine stencil), with its
+// inverse diagonal and FP32 half stencil; syncs
 // the stream once (the general-path element count)
 int launch_galerkin_fine(Ctx &c, double *Sc, cudaStream_t s);
 void launch_stencil_diag(const Level &v, const double *S, double *dinv64,
@@ -442,12 +445,6 @@ void launch_cg_update(const Ctx &c, int64_t n, T *x, T *r, const T *p,
                       cudaStream_t s, int nb = 1);
 template <typename T>
 void launch_power_start(int64_t n, T *a, cudaStream_t s);
-// w *= dinv and its squared norm (FP64 sums) into *out (the previous *out
-// into *shift_to), one pass; reduction scratch as launch_dot's
-template <typename T>
-void launch_scale_diag_dot(const Ctx &c, int64_t n, T *w, const T *dinv, double *out,
-                           double *shift_to, cudaStream_t s, double *part,
-                           unsigned int *ticket);
 void launch_to_f32_scaled(int64_t n, const double *a, const double *scal,
                           float *b, cudaStream_t s, int nb = 1);
 void launch_axpy_f32(int64_t n, double *U, const float *d, const double *scal,
