@@ -81,3 +81,38 @@ def test_eigensolver_block_sizes(T, nel, levels, nev, block):
     ref = sl.eigh(np.diag(M), K[np.ix_(free, free)], eigvals_only=True)[::-1]
     w = np.linalg.eigvalsh(K)
     assert np.allclose(lam, ref[:lam.size], rtol=n * 1.1e-16 * w[-1] / w[0] + 1e-13, atol=0)
+
+
+# the tiled filter: halos of 1 (also a radius with one tap), 2 and 3 elements
+# and the untiled form beyond, below, at and across the 32 x 16 x 4 tiles
+@pytest.mark.parametrize("rmin", [0.9, 1.5, 2.0, 2.5, 3.0, 4.0, 4.3])
+@pytest.mark.parametrize("nel", [(1, 1, 1), (3, 2, 5), (31, 16, 4), (33, 17, 9), (64, 15, 3)])
+def test_filter_matches_its_matrix(T, nel, rmin):
+    """P and P^T against the row-normalised cone summed in numpy: at most 305
+    terms of one sign pattern, so rounding stays below 305 u of sum |terms|."""
+    nx, ny, nz = nel
+    t = T.TopOpt(nel, rmin=rmin, mg_levels=1 if max(nel) < 32 else 2)
+    rng = np.random.default_rng(5)
+    n = int(rmin)
+
+    def cone(v):
+        out = np.zeros_like(v)
+        for k in range(-n, n + 1):
+            for j in range(-n, n + 1):
+                for i in range(-n, n + 1):
+                    d = np.sqrt(i * i + j * j + k * k)
+                    if d >= rmin or abs(i) >= nx or abs(j) >= ny or abs(k) >= nz:
+                        continue
+                    dst = tuple(slice(max(0, -a), m - max(0, a)) for a, m in
+                                ((k, nz), (j, ny), (i, nx)))
+                    src = tuple(slice(max(0, a), m - max(0, -a)) for a, m in
+                                ((k, nz), (j, ny), (i, nx)))
+                    out[dst] += (1.0 - d / rmin) * v[src]
+        return out
+    rows = cone(np.ones((nz, ny, nx)))
+    for transpose in (False, True):
+        v = rng.uniform(-1.0, 1.0, (nz, ny, nx))
+        ref = cone(v / rows) if transpose else cone(v) / rows
+        size = cone(np.abs(v) / rows) if transpose else cone(np.abs(v)) / rows
+        got = t.filter(v.reshape(-1), transpose=transpose).reshape(nz, ny, nx)
+        assert np.all(np.abs(got - ref) <= 2 * 305 * 1.1e-16 * size)
