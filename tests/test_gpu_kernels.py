@@ -116,3 +116,26 @@ def test_filter_matches_its_matrix(T, nel, rmin):
         size = cone(np.abs(v) / rows) if transpose else cone(np.abs(v)) / rows
         got = t.filter(v.reshape(-1), transpose=transpose).reshape(nz, ny, nx)
         assert np.all(np.abs(got - ref) <= 2 * 305 * 1.1e-16 * size)
+
+
+# the OC bisection keeps its elements in registers on few blocks: part of a
+# block, exactly one and one element more, exactly one element a thread on 148
+# blocks (151,552), past it, exactly two, past that (the arrays read again)
+@pytest.mark.parametrize("nel", [(13, 6, 6), (16, 8, 8), (41, 5, 5), (64, 37, 64), (64, 37, 65),
+                                 (128, 37, 64), (64, 75, 65)])
+def test_oc_update_over_sizes(T, oracle, nel):
+    """The bisection against the oracle's: the same branches, so what differs is
+    rounding (1e-16 a term; the last multiplier interval, 1e-9 of the
+    multiplier, moves the constraint sum 1e5 times more than its rounding)."""
+    n = int(np.prod(nel))
+    t = T.TopOpt(nel, mg_levels=2 if n < 2000 else 4)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0.2, 0.8, n)
+    dfdx = -rng.uniform(0.0, 1.0, n)
+    dfdx[::7] = 0.3
+    dgdx = rng.uniform(0.5, 1.5, n) / n
+    oc = T.OC(n, move=0.2)
+    oc.xval = x.copy()
+    xg = oc.Update(t, dfdx.copy(), np.array([0.02]), dgdx[:, None])
+    xo, cho = oracle.oc_update(x, dfdx, 0.02, dgdx, 0.2)
+    assert np.max(np.abs(xg - xo)) < 1e-12 and abs(oc.Change - cho) < 1e-12

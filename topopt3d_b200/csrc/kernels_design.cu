@@ -240,8 +240,34 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// one bisection trial of MMA::OCsub (MMA.cpp:139-160): candidate x and
-// per-block partial sums of dgdx . (x - xold)
+// One element of a bisection trial of MMA::OCsub (MMA.cpp:139-160).  What the
+// multiplier does not change is formed once: ratio = -dfdx / dgdx, the
+// distance to xmin, and the bounds the clamp sequence min(xold + step), min
+// (xmax), max(xold - step), max(xmin) comes down to.
+struct OcElem {
+  double ratio, lo, dist, top, bottom, dg, xo;
+  __device__ __forceinline__ void load(int64_t i, const double *xold, const double *xmin,
+                                       const double *xmax, const double *dfdx,
+                                       const double *dgdx, double move) {
+    xo = xold[i];
+    lo = xmin[i];
+    const double hi = xmax[i], step = move * (hi - lo);
+    dg = dgdx[i];
+    ratio = -dfdx[i] / dg;
+    if (isinf(ratio)) ratio = fabs(ratio);   // dg = -0: as the power 1/2 has it
+    dist = xo - lo;
+    top = fmin(xo + step, hi);
+    bottom = fmax(xo - step, lo);
+  }
+  // the candidate x; adds dgdx (x - xold) to s
+  __device__ __forceinline__ double trial(double lmid, double &s) const {
+    const double v = fmax(fmin(lo + dist * sqrt(ratio / lmid), top), bottom);
+    s += dg * (v - xo);
+    return v;
+  }
+};
+
+// one trial: candidate x and per-block partial sums of dgdx . (x - xold)
 __global__ void k_oc_step(int64_t n, double *x, const double *xold,
                           const double *xmin, const double *xmax,
                           const double *dfdx, const double *dgdx, double move,
@@ -250,16 +276,9 @@ __global__ void k_oc_step(int64_t n, double *x, const double *xold,
   double s = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const double B = pow(-dfdx[i] / dgdx[i] / lmid, 0.5);
-    const double xo = xold[i], lo = xmin[i], hi = xmax[i];
-    const double step = move * (hi - lo);
-    double v = lo + (xo - lo) * B;
-    v = fmin(v, xo + step);
-    v = fmin(v, hi);
-    v = fmax(v, xo - step);
-    v = fmax(v, lo);
-    x[i] = v;
-    s += dgdx[i] * (v - xo);
+    OcElem el;
+    el.load(i, xold, xmin, xmax, dfdx, dgdx, move);
+    x[i] = el.trial(lmid, s);
   }
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
@@ -286,64 +305,73 @@ __global__ void k_sum_parts(int nparts, const double *part, double *out) {
 }
 
 // The whole bisection of MMA::OCsub (MMA.cpp:136-161) in one cooperative
-// launch of kRedBlocks x 256 threads, with no host round trip per trial.
-// Each trial forms the candidate x and the block's partial of
-// dgdx . (x - xold) exactly as k_oc_step does on the same grid; after a grid
-// barrier every block sums the kRedBlocks partials in k_sum_parts' order,
-// so all blocks hold the same total and take the same branch.  The
-// partials are double-buffered by trial parity: a block writes the next
-// trial's partials only after the next barrier, which every block reaches
-// after reading the current ones.
-__global__ void __launch_bounds__(256)
+// launch, with no host round trip per trial.  Each trial forms the candidate
+// x and the block's partial of dgdx . (x - xold); after a grid barrier every
+// block sums the partials in the same order, so all blocks hold the same
+// total and take the same branch.  The partials are double-buffered by trial
+// parity: a block writes the next trial's partials only after the next
+// barrier, which every block reaches after reading the current ones.
+// A trial is latency: its square root and divide, two block sums and the
+// barrier.  With EPT > 0 a thread keeps its EPT elements in registers for all
+// trials, on as few blocks as that takes (EPT = 0: any n, the arrays are read
+// again).  The update of 432 elements from host arrays takes 144 us (213 us
+// with the arrays and a power read on every trial), of 65,536 550 us (604 us),
+// most of it then the copies; the kernel of the latter 90 us.
+constexpr int kOcThreads = 1024;
+template <int EPT>
+__global__ void __launch_bounds__(kOcThreads, 1)
     k_oc_bisect(int64_t n, double *x, const double *xold, const double *xmin,
                 const double *xmax, const double *dfdx, const double *dgdx,
                 double move, double g, double *part, unsigned int *bar,
                 double *fault) {
   __shared__ double sh[32];
   __shared__ double total;
+  unsigned int sense = grid_barrier_sense(bar);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = gridDim.x;
+  const int64_t i0 = blockIdx.x * (int64_t)kOcThreads + threadIdx.x;
+  const int64_t di = (int64_t)G * kOcThreads;
+  OcElem el[EPT > 0 ? EPT : 1];
+#pragma unroll
+  for (int u = 0; u < EPT; ++u)
+    if (i0 + u * di < n) el[u].load(i0 + u * di, xold, xmin, xmax, dfdx, dgdx, move);
+  double xv[EPT > 0 ? EPT : 1];
   double l1 = 0, l2 = 1e6;
   int trial = 0;
   while (l2 - l1 > 1e-4) {
     const double lmid = 0.5 * (l1 + l2);
-    double *pp = part + (trial & 1) * gridDim.x;
+    double *pp = part + (trial & 1) * G;
     double s = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const double B = pow(-dfdx[i] / dgdx[i] / lmid, 0.5);
-      const double xo = xold[i], lo = xmin[i], hi = xmax[i];
-      const double step = move * (hi - lo);
-      double v = lo + (xo - lo) * B;
-      v = fmin(v, xo + step);
-      v = fmin(v, hi);
-      v = fmax(v, xo - step);
-      v = fmax(v, lo);
-      x[i] = v;
-      s += dgdx[i] * (v - xo);
+    if (EPT > 0) {
+#pragma unroll
+      for (int u = 0; u < EPT; ++u)
+        if (i0 + u * di < n) xv[u] = el[u].trial(lmid, s);
+    } else {
+      for (int64_t i = i0; i < n; i += di) {
+        el[0].load(i, xold, xmin, xmax, dfdx, dgdx, move);
+        x[i] = el[0].trial(lmid, s);
+      }
     }
     s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    if (lane == 0) sh[w] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-      s = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
-      s = warp_sum(s);
-      if (threadIdx.x == 0) pp[blockIdx.x] = s;
+    if (w == 0) {
+      s = warp_sum(sh[lane]);
+      if (lane == 0) pp[blockIdx.x] = s;
     }
-    if (!grid_barrier(bar, fault)) return;
-    double t = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += pp[i];
-    t = warp_sum(t);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      t = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
+    if (!grid_barrier_red(bar, fault, &sense)) return;
+    if (w == 0) {
+      double t = 0;
+      for (int i = lane; i < G; i += 32) t += __ldcg(pp + i);
       t = warp_sum(t);
-      if (threadIdx.x == 0) total = t;
+      if (lane == 0) total = t;
     }
     __syncthreads();
     if (g + total > 0) l1 = lmid; else l2 = lmid;
     ++trial;
-    __syncthreads();
   }
+#pragma unroll
+  for (int u = 0; u < EPT; ++u)
+    if (i0 + u * di < n) x[i0 + u * di] = xv[u];
 }
 
 // ---- MMA for m >= 2 constraints (MMA::MMAsub, MMA.cpp:185-343, with
@@ -788,27 +816,38 @@ void launch_oc_step(const Ctx &c, int64_t n, double *x, const double *xold,
   k_sum_parts<<<1, 256, 0, s>>>(kRedBlocks, c.part, out);
 }
 
+template <int EPT>
+static cudaError_t oc_bisect(int grid, void **args, cudaStream_t s) {
+  return cudaLaunchCooperativeKernel((const void *)k_oc_bisect<EPT>, grid, kOcThreads, args, 0, s);
+}
+
 bool launch_oc_bisect(const Ctx &c, int64_t n, double *x, const double *xold,
                       const double *xmin, const double *xmax, const double *dfdx,
                       const double *dgdx, double move, double g, cudaStream_t s,
                       cudaError_t *err) {
-  static int fits[64] = {0};   // 1: kRedBlocks co-resident CTAs fit, -1: not
+  static int ctas[64] = {0};   // co-resident CTAs (one per SM), -1: none
   int dev = 0;
   cudaGetDevice(&dev);
   dev &= 63;
-  if (!fits[dev]) {
+  if (!ctas[dev]) {
     int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oc_bisect, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oc_bisect<2>, kOcThreads, 0);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    fits[dev] = per_sm * sms >= kRedBlocks ? 1 : -1;
+    ctas[dev] = per_sm > 0 ? std::min(sms, kRedBlocks) : -1;
   }
-  if (fits[dev] < 0) return false;
+  if (ctas[dev] < 0) return false;
   count_launch();
   double *part = c.part;   // 2 x kRedBlocks <= kPartCount
   unsigned int *bar = c.gbar;
   double *fault = c.scal + kSlotFault;
   void *args[] = {&n, &x, &xold, &xmin, &xmax, &dfdx, &dgdx, &move, &g, &part, &bar, &fault};
-  *err = cudaLaunchCooperativeKernel((const void *)k_oc_bisect, kRedBlocks, 256, args, 0, s);
+  const int64_t full = (int64_t)ctas[dev] * kOcThreads;
+  const int ept = n <= full ? 1 : (n <= 2 * full ? 2 : 0);
+  const int64_t per = (int64_t)kOcThreads * (ept ? ept : 1);
+  const int grid = (int)std::min<int64_t>((n + per - 1) / per, ctas[dev]);
+  *err = ept == 1   ? oc_bisect<1>(grid, args, s)
+         : ept == 2 ? oc_bisect<2>(grid, args, s)
+                    : oc_bisect<0>(grid, args, s);
   return true;
 }
 
