@@ -139,3 +139,18 @@ def test_oc_update_over_sizes(T, oracle, nel):
     xg = oc.Update(t, dfdx.copy(), np.array([0.02]), dgdx[:, None])
     xo, cho = oracle.oc_update(x, dfdx, 0.02, dgdx, 0.2)
     assert np.max(np.abs(xg - xo)) < 1e-12 and abs(oc.Change - cho) < 1e-12
+
+
+# the z chunks of the matrix-free operator, from one plane to all: a block of
+# columns cuts z at other planes than one column does
+@pytest.mark.parametrize("nel", [(1, 1, 1), (12, 6, 6), (5, 9, 30), (30, 7, 17), (48, 24, 24)])
+def test_apply_chunks_give_the_same_values(T, nel):
+    """A node's value does not depend on the chunk it is in, bit for bit."""
+    t = make(T, nel, 1 if int(np.prod(nel)) < 2000 else 3, assemble=False)
+    n, nb = 3 * t.nNode, 40
+    u = np.random.default_rng(1).standard_normal(nb * n)
+    y, y1 = np.zeros_like(u), np.zeros(n)
+    t.apply(u, y, nrhs=nb)
+    for j in (0, nb - 1):
+        t.apply(u[j * n:(j + 1) * n], y1)
+        assert np.array_equal(y1, y[j * n:(j + 1) * n])

@@ -463,16 +463,24 @@ void set_smem_attr() {
 }
 
 // grid of the staged kernel: 30 x (kTY-1) owned node columns per CTA, and z
-// chunks that fill whole waves of co-resident CTAs (a partial last wave
-// idles SMs for the length of a chunk; each chunk recomputes one element
-// layer and two face planes)
+// chunks chosen by their time: a CTA takes its planes and about 2.3 more (the
+// pipeline's fill, and the element layer a chunk computes again), 0.85 us
+// (FP64) or 0.6 us (FP32) each, and the CTAs run in waves of what the SMs
+// hold -- one an SM in FP64; two in FP32, which share it: the pair's planes
+// take 1.55 times as long as one CTA's alone.  Against the best of all chunk
+// counts, measured for ten meshes from 12x6x6 to 192x96x96 in FP32, FP64 and
+// blocks of 5 and 8 columns, this choice is 0.3% slower in the mean, at most
+// 9%.  Chunks of at least 8 planes in whole waves took, in us: 10.4 (now 5.5)
+// for 12x6x6, 12.5 (6.4) for 48x24x24, 14.6 (14.6) for 91x47x53 and 29.9
+// (27.0) for 128x64x64 in FP64; 12.6 (10.4) and 18.6 (16.6) for the last two
+// in FP32.
 template <typename T>
 void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
   const int Nx = c.nel[0] + 1, Ny = c.nel[1] + 1, Nz = c.nel[2] + 1;
   const int gx = (Nx + kLanesOut - 1) / kLanesOut, gy = (Ny + kTY - 2) / (kTY - 1);
   const int dev = c.device & 63;
   static unsigned long long attr_set = 0;   // bit per device
-  static int slots_cache[64] = {0};
+  static int slots_cache[64] = {0}, sms_cache[64] = {0};
   if (!((attr_set >> dev) & 1ull)) {
     // opt in to > 48 KB of dynamic shared memory (the FP64 tiles)
     set_smem_attr<T, IN_U, OUT_Y>();
@@ -486,21 +494,25 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
         &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true>, 32 * kTY,
         staged_smem<T, IN_CHEB, OUT_CHEB2>());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    slots_cache[dev] = std::max(1, per_sm) * std::max(1, sms);
+    sms_cache[dev] = std::max(1, sms);
+    slots_cache[dev] = std::max(1, per_sm) * sms_cache[dev];
     attr_set |= 1ull << dev;
   }
-  const int slots = slots_cache[dev], tiles = gx * gy * nb;
+  const int slots = slots_cache[dev], sms = sms_cache[dev], tiles = gx * gy * nb;
+  double best = 0;
   int chunks = 1;
-  for (int w = 1; w <= 8; ++w) {
-    const int ch = (w * slots) / tiles;
-    if (ch >= 1 && (double)(ch * tiles) >= 0.9 * w * slots) {
+  // beyond four waves more chunks only add planes
+  for (int ch = 1; ch <= Nz && (ch == 1 || (int64_t)ch * tiles <= 4 * (int64_t)slots); ++ch) {
+    const int zc = (Nz + ch - 1) / ch;
+    const int64_t n = (int64_t)tiles * ((Nz + zc - 1) / zc), rest = n % slots;
+    const double shared = slots > sms ? 1.55 : 1.0;
+    const double waves = shared * (double)(n / slots) + (rest == 0 ? 0.0 : rest <= sms ? 1.0 : shared);
+    const double t = waves * (zc + 2.3);
+    if (ch == 1 || t < best) {
+      best = t;
       chunks = ch;
-      break;
     }
-    chunks = std::max(1, ch);
   }
-  const int maxc = std::max(1, Nz / 8);   // keep >= 8 planes per chunk
-  if (chunks > maxc) chunks = maxc;
   zchunk = (Nz + chunks - 1) / chunks;
   grid = dim3(gx, gy, nb * ((Nz + zchunk - 1) / zchunk));
 }
