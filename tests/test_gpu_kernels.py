@@ -154,3 +154,31 @@ def test_apply_chunks_give_the_same_values(T, nel):
     for j in (0, nb - 1):
         t.apply(u[j * n:(j + 1) * n], y1)
         assert np.array_equal(y1, y[j * n:(j + 1) * n])
+
+
+# CG's dot products: in the operator's epilogue (degree 2), by a pass of their
+# own (other degrees, one level), one column and blocks of 3 and 8, on meshes of
+# one CTA and of many
+@pytest.mark.parametrize("nel,levels", [((4, 3, 2), 1), ((12, 6, 6), 2), ((31, 14, 9), 3)])
+@pytest.mark.parametrize("degree", [1, 2, 3])
+@pytest.mark.parametrize("nb", [1, 3, 8])
+def test_cg_dot_products(T, nel, levels, degree, nb):
+    """Every column ends below its target, and no sooner than CG has to: the
+    same iterations as the column alone (a sum in another order moves ||r|| by
+    1e-14 of itself, an iteration moves it by tenths)."""
+    o = T.default_opts(cheb_degree=degree, rtol=1e-6, precision=T.PREC_FP64)
+    t = make(T, nel, levels, opts=o)
+    n = 3 * t.nNode
+    b = np.random.default_rng(2).standard_normal((nb, n))
+    fm, _ = t.get_bc()
+    b[:, [d for d in range(n) if (fm[d // 3] >> (d % 3)) & 1]] = 0.0
+    U, y = np.zeros_like(b), np.zeros_like(b)
+    its = t.solve(b, U, nrhs=nb, opts=o)["iterations"]
+    t.apply(U, y, nrhs=nb)
+    assert np.all(np.linalg.norm(b - y, axis=1) <= 1.0001e-6 * np.linalg.norm(b, axis=1))
+    alone = []
+    for j in range(nb):
+        Uj = np.zeros(n)
+        alone.append(t.solve(b[j].copy(), Uj, opts=o)["iterations"])
+        assert np.linalg.norm(Uj - U[j]) <= 1e-5 * np.linalg.norm(Uj)
+    assert its == sum(alone)

@@ -270,7 +270,7 @@ void free_all(Ctx &c) {
   if (c.mma_h) cudaFreeHost(c.mma_h);
   c.mma_h = nullptr; dfree(c.ks_S); dfree(c.ks_H); dfree(c.eig_buf);
   c.eig_n = 0;
-  dfree(c.scal); dfree(c.part); dfree(c.ticket); dfree(c.gbar); dfree(c.tmpe); dfree(c.tmpe2);
+  dfree(c.scal); dfree(c.part); c.apply_part = nullptr; dfree(c.ticket); dfree(c.gbar); dfree(c.tmpe); dfree(c.tmpe2);
   dfree(c.io_a); dfree(c.io_b);
   dfree(c.oc_ws);
   if (c.scal_h) cudaFreeHost(c.scal_h);
@@ -472,7 +472,11 @@ int tpo_create(const tpo_mesh_params *p, tpo_ctx **out) {
     A(c.l1_count, 1); A(c.l1_fault, 1);
   }
   A(c.fix, c.nn); A(c.idm, c.nn); A(c.F, 3 * c.nn); A(c.U, 3 * c.nn);
-  A(c.scal, tpo::kScalCount); A(c.part, tpo::kPartCount); A(c.ticket, tpo::kMaxBatch + tpo::kAuxStreams);
+  A(c.scal, tpo::kScalCount); A(c.ticket, tpo::kMaxBatch + tpo::kAuxStreams);
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+  A(c.part, tpo::kPartCount + tpo::apply_dot_parts(c.nel, sms));
+  c.apply_part = c.part + tpo::kPartCount;
   A(c.gbar, 1);
   A(c.tmpe, c.ne); A(c.tmpe2, c.ne); A(c.dev_info, 1);
   A(c.io_a, nio); A(c.io_b, nio);

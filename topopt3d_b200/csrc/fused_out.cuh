@@ -18,27 +18,28 @@ __device__ __forceinline__ T sym_in(const ApplyArgs<T> &a, int i) {
 }
 
 // the epilogue on values already loaded: bi = b[i], di = dinv[i],
-// y2i = y2[i] (each read only by the forms that use it)
+// y2i = y2[i] (each read only by the forms that use it); returns y[i]
 template <typename T, int OUT, typename I>
-__device__ __forceinline__ void sym_out_v(const ApplyArgs<T> &a, I i, T Au, T u, T bi, T di,
-                                          T y2i) {
+__device__ __forceinline__ T sym_out_v(const ApplyArgs<T> &a, I i, T Au, T u, T bi, T di, T y2i) {
+  T y;
   if (OUT == OUT_Y) {
-    a.y[i] = Au;
+    y = Au;
   } else if (OUT == OUT_RESID) {
-    a.y[i] = bi - Au;
+    y = bi - Au;
   } else if (OUT == OUT_CHEB2) {
     const T r1 = di * bi - di * Au;
-    a.y[i] = u + (a.c1 * u + a.c2 * r1);
+    y = u + (a.c1 * u + a.c2 * r1);
   } else if (OUT == OUT_POST0) {
-    const T d0 = a.invtheta * (di * (bi - Au));
-    a.y[i] = d0;
-    a.y2[i] = u + d0;
+    y = a.invtheta * (di * (bi - Au));
+    a.y2[i] = u + y;
   } else if (OUT == OUT_SCALE) {
-    a.y[i] = Au * di;
+    y = Au * di;
   } else {   // OUT_POST1
     const T r1 = a.theta * u - di * Au;
-    a.y[i] = y2i + (a.c1 * u + a.c2 * r1);
+    y = y2i + (a.c1 * u + a.c2 * r1);
   }
+  a.y[i] = y;
+  return y;
 }
 
 template <int OUT>

@@ -38,6 +38,7 @@
 // complete, and nodes of plane p-2 are written.
 #include "fused_out.cuh"
 #include "modal.cuh"
+#include "reduce.cuh"
 
 namespace tpo {
 
@@ -87,12 +88,14 @@ __device__ __forceinline__ void copy_wait() {
 // staged arrays and planes: IN_CHEB keeps b and dinv of 4 planes (loaded
 // ahead, input, and two planes later the epilogue) and the row above the
 // tile; the other forms 2 planes of what their epilogue reads; the
-// Chebyshev forms with IN_U also keep their input of 3 planes (4 slots)
-template <int IN, int OUT>
+// Chebyshev forms with IN_U, and the product whose dot with u is formed, also
+// keep their input of 3 planes (4 slots)
+template <int IN, int OUT, bool DOT>
 struct Staged {
   static constexpr bool kIn = IN == IN_CHEB;
-  static constexpr bool kB = OutNeeds<OUT>::b, kD = OutNeeds<OUT>::dinv, kY = OutNeeds<OUT>::y2;
-  static constexpr bool kU = !kIn && (OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1);
+  static constexpr bool kB = OutNeeds<OUT>::b || (DOT && OUT == OUT_POST1), kD = OutNeeds<OUT>::dinv, kY = OutNeeds<OUT>::y2;
+  static constexpr bool kU = !kIn && (OUT == OUT_CHEB2 || OUT == OUT_POST0 || OUT == OUT_POST1 ||
+                                      (DOT && OUT == OUT_Y));
   static constexpr int kArrays = kIn ? 2 : int(kB) + int(kD) + int(kY);
   static constexpr int kSlots = kIn ? 4 : 2;
   static constexpr int kSlotB = 0, kSlotD = kIn ? 1 : int(kB), kSlotY = int(kB) + int(kD);
@@ -155,11 +158,17 @@ struct Six<double> {
 // COLS: a block of columns, blockIdx.z = column * nchunk + z chunk, the
 // column selecting u, b, y, y2 (stride ld).  The single-column
 // instantiation reads the parameters in place.
-template <typename T, int TY, int IN, int OUT, bool COLS>
+//
+// DOT: the epilogue also sums, in FP64, u.y (OUT_Y), y.y (OUT_RESID) or b.y
+// (OUT_POST1): CG's p.q, r.r of a replaced residual and rho = r.z.  A pass of
+// its own that reads both vectors again took 11 us in FP32 and 19 us in FP64 at
+// 192x96x96 (6 us at 48x24x24); here p.q adds 4 and 6 us, rho 5 and 6.5 us (a
+// third staged operand), r.r 4 us (FP64), most of it in FP32 the conversions.
+template <typename T, int TY, int IN, int OUT, bool COLS, bool DOT>
 __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     k_apply_staged(int nelx, int nely, int nelz, int zchunk,
                    const T *__restrict__ E, const uint8_t *__restrict__ fix,
-                   const ApplyArgs<T> args_in, const Kh<T> kh) {
+                   const ApplyArgs<T> args_in, const Kh<T> kh, const DotOut dot) {
   const int Nx = nelx + 1, Ny = nely + 1, Nz = nelz + 1;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int gx = (int)blockIdx.x * kLanesOut - 1 + tx;
@@ -205,7 +214,7 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
 
   // the staged operands, 3 values per thread: element (array, slot, row,
   // lane, component)
-  using Sg = Staged<IN, OUT>;
+  using Sg = Staged<IN, OUT, DOT>;
   T *stage = reinterpret_cast<T *>(smem_raw + 4 * kRows * Six<T>::bytes_per_row());
   auto slot_at = [&](int arr, int z, int row) -> T * {
     return stage + ((arr * Sg::kSlots + (z & (Sg::kSlots - 1))) * kRows + row) * 96 + 3 * tx;
@@ -282,6 +291,7 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     for (int c = 0; c < 3; ++c) FA[m][c] = FB[m][c] = CA[m][c] = CB[m][c] = T(0);
 #pragma unroll
   for (int c = 0; c < 3; ++c) les[c] = led[c] = T(0);
+  double dsum = 0;       // this thread's share of the dot product
   unsigned fpipe = 0u;   // fixed bits of the last three planes, 8 bits each
 
   // one step of the z-march at plane p: Fprev = faces of plane p-1 (in),
@@ -383,7 +393,10 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
             uv = su[c];
           else if (fixed)
             uv = __ldg(args.u + i + c);
-          sym_out_v<T, OUT>(args, i + c, fixed ? uv : val[c], uv, bi, di, yi);
+          const T yv = sym_out_v<T, OUT>(args, i + c, fixed ? uv : val[c], uv, bi, di, yi);
+          if (DOT)
+            dsum += static_cast<double>(OUT == OUT_Y ? uv : OUT == OUT_RESID ? yv : bi) *
+                    static_cast<double>(yv);
         }
       }
     }
@@ -443,23 +456,33 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     step(p, FA, FB, CA, CB);
     if (p + 1 <= ze + 1) step(p + 1, FB, FA, CB, CA);
   }
+  if (DOT) {
+    // one partial per CTA of the column
+    const int nchunk = args_in.nchunk, col = COLS ? (int)blockIdx.z / nchunk : 0;
+    if (dot.skip && dot.skip[col * kColScal] != 0.0) return;
+    const int per = gridDim.x * gridDim.y * nchunk;
+    const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * (blockIdx.z - col * nchunk));
+    finish_reduction(dsum, ty * 32 + tx, 32 * TY, cta, per, dot.part + (int64_t)col * per,
+                     dot.ticket + col, dot.out + col * kColScal,
+                     dot.shift ? dot.shift + col * kColScal : nullptr);
+  }
 }
 
 constexpr int kTY = 8;
 
-template <typename T, int IN, int OUT>
+template <typename T, int IN, int OUT, bool DOT>
 constexpr size_t staged_smem() {
-  return (kTY + 1) * (4 * Six<T>::bytes_per_row() + Staged<IN, OUT>::planes() * 96 * sizeof(T));
+  return (kTY + 1) * (4 * Six<T>::bytes_per_row() + Staged<IN, OUT, DOT>::planes() * 96 * sizeof(T));
 }
 
-template <typename T, int IN, int OUT>
+template <typename T, int IN, int OUT, bool DOT = false>
 void set_smem_attr() {
-  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, false>,
+  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, false, DOT>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)staged_smem<T, IN, OUT>());
-  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, true>,
+                       (int)staged_smem<T, IN, OUT, DOT>());
+  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, true, DOT>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)staged_smem<T, IN, OUT>());
+                       (int)staged_smem<T, IN, OUT, DOT>());
 }
 
 // grid of the staged kernel: 30 x (kTY-1) owned node columns per CTA, and z
@@ -489,10 +512,13 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
     set_smem_attr<T, IN_U, OUT_POST0>();
     set_smem_attr<T, IN_U, OUT_POST1>();
     set_smem_attr<T, IN_U, OUT_SCALE>();
+    set_smem_attr<T, IN_U, OUT_Y, true>();
+    set_smem_attr<T, IN_U, OUT_RESID, true>();
+    set_smem_attr<T, IN_U, OUT_POST1, true>();
     int per_sm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true>, 32 * kTY,
-        staged_smem<T, IN_CHEB, OUT_CHEB2>());
+        &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true, false>, 32 * kTY,
+        staged_smem<T, IN_CHEB, OUT_CHEB2, false>());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
     sms_cache[dev] = std::max(1, sms);
     slots_cache[dev] = std::max(1, per_sm) * sms_cache[dev];
@@ -517,48 +543,65 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
   grid = dim3(gx, gy, nb * ((Nz + zchunk - 1) / zchunk));
 }
 
-template <typename T, int IN, int OUT>
+template <typename T, int IN, int OUT, bool DOT = false>
 void launch_mode(const Ctx &c, const T *E, const ApplyArgs<T> &args_in,
-                 cudaStream_t s, int nb) {
+                 cudaStream_t s, int nb, DotOut dot = {}) {
   dim3 grid;
   int zchunk = 0;
   staged_grid<T>(c, nb, grid, zchunk);
   ApplyArgs<T> args = args_in;
   args.ld = 3 * c.nn;
   args.nchunk = (int)grid.z / nb;
+  dot.part = c.apply_part;
+  dot.ticket = c.ticket;
   const Kh<T> &kh = *reinterpret_cast<const Kh<T> *>(
       sizeof(T) == 8 ? (const void *)&c.kh64 : (const void *)&c.kh32);
+  constexpr size_t smem = staged_smem<T, IN, OUT, DOT>();
   count_launch();
   if (nb == 1)
-    k_apply_staged<T, kTY, IN, OUT, false><<<grid, dim3(32, kTY), staged_smem<T, IN, OUT>(), s>>>(
-        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh);
+    k_apply_staged<T, kTY, IN, OUT, false, DOT><<<grid, dim3(32, kTY), smem, s>>>(
+        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
   else
-    k_apply_staged<T, kTY, IN, OUT, true><<<grid, dim3(32, kTY), staged_smem<T, IN, OUT>(), s>>>(
-        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh);
+    k_apply_staged<T, kTY, IN, OUT, true, DOT><<<grid, dim3(32, kTY), smem, s>>>(
+        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
 }
 
 }  // namespace
 
+// staged_grid makes at most max(4 x resident CTAs, tiles x columns) CTAs
+int64_t apply_dot_parts(const int *nel, int sms) {
+  const int64_t gx = (nel[0] + 1 + kLanesOut - 1) / kLanesOut;
+  const int64_t gy = (nel[1] + 1 + kTY - 2) / (kTY - 1);
+  constexpr int kMaxPerSm = 2048 / (32 * kTY);
+  return std::max<int64_t>(4 * kMaxPerSm * (int64_t)sms, gx * gy * kMaxBatch);
+}
+
 template <typename T>
 void launch_apply_fine(const Ctx &c, const T *E, const T *u, const T *b, T *y,
-                       cudaStream_t s, int nb) {
+                       cudaStream_t s, int nb, const DotOut *dot) {
   ApplyArgs<T> a{};
   a.u = u;
   a.b = b;
   a.y = y;
-  if (b)
+  if (b && dot)
+    launch_mode<T, IN_U, OUT_RESID, true>(c, E, a, s, nb, *dot);
+  else if (b)
     launch_mode<T, IN_U, OUT_RESID>(c, E, a, s, nb);
+  else if (dot)
+    launch_mode<T, IN_U, OUT_Y, true>(c, E, a, s, nb, *dot);
   else
     launch_mode<T, IN_U, OUT_Y>(c, E, a, s, nb);
 }
 
 template <typename T>
 void launch_apply_fused(const Ctx &c, const T *E, int in, int out,
-                        const ApplyArgs<T> &args, cudaStream_t s, int nb) {
+                        const ApplyArgs<T> &args, cudaStream_t s, int nb, const DotOut *dot) {
   if (in == IN_CHEB && out == OUT_CHEB2)
     launch_mode<T, IN_CHEB, OUT_CHEB2>(c, E, args, s, nb);
   else if (in == IN_U && out == OUT_POST0)
     launch_mode<T, IN_U, OUT_POST0>(c, E, args, s, nb);
+  else if (in == IN_U && out == OUT_POST1 && dot)
+    launch_mode<T, IN_U, OUT_POST1, true>(c, E, args, s, nb, *dot);
   else if (in == IN_U && out == OUT_POST1)
     launch_mode<T, IN_U, OUT_POST1>(c, E, args, s, nb);
   else if (in == IN_U && out == OUT_RESID)
@@ -571,15 +614,15 @@ void launch_apply_fused(const Ctx &c, const T *E, int in, int out,
 
 template void launch_apply_fine<double>(const Ctx &, const double *,
                                         const double *, const double *,
-                                        double *, cudaStream_t, int);
+                                        double *, cudaStream_t, int, const DotOut *);
 template void launch_apply_fine<float>(const Ctx &, const float *,
                                        const float *, const float *, float *,
-                                       cudaStream_t, int);
+                                       cudaStream_t, int, const DotOut *);
 template void launch_apply_fused<double>(const Ctx &, const double *, int, int,
                                          const ApplyArgs<double> &,
-                                         cudaStream_t, int);
+                                         cudaStream_t, int, const DotOut *);
 template void launch_apply_fused<float>(const Ctx &, const float *, int, int,
                                         const ApplyArgs<float> &, cudaStream_t,
-                                        int);
+                                        int, const DotOut *);
 
 }  // namespace tpo

@@ -1,11 +1,12 @@
 // Vector kernels of the Krylov solvers.  Every reduction accumulates in FP64
-// and is deterministic: a fixed grid of kRedBlocks blocks writes one partial
-// each in a fixed order, and the last block to finish (ticket counter) sums
+// and is deterministic: a grid fixed by the length (red_grid) writes one partial
+// per block in a fixed order, and the last block to finish (ticket counter) sums
 // the partials in a fixed tree order and writes the result to a device
 // scalar, so the CG recurrences never round-trip through the host.
 #include <algorithm>
 #include <cstdint>
 
+#include "reduce.cuh"
 #include "tpo_internal.h"
 
 namespace tpo {
@@ -19,50 +20,6 @@ int grid_for(int64_t n, int threads) {
   if (g > 148 * 32) g = 148 * 32;
   if (g < 1) g = 1;
   return (int)g;
-}
-
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  v = 0;
-  if (threadIdx.x < 32) {
-    v = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  }
-  __syncthreads();
-  return v;   // valid in thread 0
-}
-
-// partial -> last block -> *out (previous *out moved to *shift_to if set).
-// Column j of a block reduction owns blocks (*, j): part + j * gridDim.x
-// and ticket + j.
-__device__ __forceinline__ void finish_reduction(double v, double *part,
-                                                 unsigned int *ticket,
-                                                 double *out, double *shift_to) {
-  __shared__ double sh[32];
-  __shared__ bool last;
-  v = block_sum(v, sh);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = v;
-    __threadfence();
-    last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double s = 0;
-  for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x)
-    s += ((volatile double *)part)[i];
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) {
-    if (shift_to) *shift_to = *out;
-    *out = s;
-    *ticket = 0u;
-  }
 }
 
 // 16-byte vectors of the streamed kernels: 4 floats or 2 doubles
@@ -129,7 +86,8 @@ __global__ void __launch_bounds__(kRedThreads)
   }
   for (int64_t i = tail + t0; i < n; i += st)
     s += static_cast<double>(a[i]) * static_cast<double>(b[i]);
-  finish_reduction(s, part + j * gridDim.x, ticket + j, out + j * kColScal,
+  finish_reduction(s, threadIdx.x, blockDim.x, blockIdx.x, gridDim.x, part + j * gridDim.x,
+                   ticket + j, out + j * kColScal,
                    shift_to ? shift_to + j * kColScal : nullptr);
 }
 
@@ -223,7 +181,8 @@ __global__ void __launch_bounds__(kRedThreads)
     }
     s += static_cast<double>(ri) * static_cast<double>(ri);
   }
-  finish_reduction(s, part + j * gridDim.x, ticket + j, rr + j * kColScal,
+  finish_reduction(s, threadIdx.x, blockDim.x, blockIdx.x, gridDim.x, part + j * gridDim.x,
+                   ticket + j, rr + j * kColScal,
                    nullptr);
 }
 
@@ -300,7 +259,7 @@ void launch_dot(const Ctx &c, int64_t n, const T *a, const T *b, double *out,
                 double *shift_to, cudaStream_t s, int nb, double *part,
                 unsigned int *ticket) {
   count_launch();
-  k_dot<T><<<dim3(red_grid(nb), nb), kRedThreads, 0, s>>>(
+  k_dot<T><<<dim3(red_grid(n, nb), nb), kRedThreads, 0, s>>>(
       n, a, b, part ? part : c.part, ticket ? ticket : c.ticket, out, shift_to,
       nullptr);
 }
@@ -309,7 +268,7 @@ template <typename T>
 void launch_rho_dot(const Ctx &c, int64_t n, const T *r, const T *z, cudaStream_t s,
                     int nb) {
   count_launch();
-  k_dot<T><<<dim3(red_grid(nb), nb), kRedThreads, 0, s>>>(
+  k_dot<T><<<dim3(red_grid(n, nb), nb), kRedThreads, 0, s>>>(
       n, r, z, c.part, c.ticket, c.scal + 0, c.scal + 1, c.scal + 6);
 }
 template void launch_rho_dot<double>(const Ctx &, int64_t, const double *,
@@ -339,7 +298,7 @@ void launch_cg_update(const Ctx &c, int64_t n, T *x, T *r, const T *p,
                       const T *q, const double *scal, double *rr,
                       cudaStream_t s, int nb) {
   count_launch();
-  k_cg_update<T><<<dim3(red_grid(nb), nb), kRedThreads, 0, s>>>(
+  k_cg_update<T><<<dim3(red_grid(n, nb), nb), kRedThreads, 0, s>>>(
       n, x, r, p, q, scal, c.part, c.ticket, rr);
 }
 template void launch_cg_update<double>(const Ctx &, int64_t, double *,

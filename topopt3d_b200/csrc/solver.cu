@@ -155,11 +155,14 @@ void prolong_from(Ctx &c, int l, T *x, cudaStream_t s, int nb) {
   launch_prolong_add<T>(v, cv, lv(cv, (T *)nullptr).x, x, comp_level(c, l + 1), s, nb);
 }
 
+// one V-cycle from level l; rho (level 0 only): with the dot product b.x of
+// CG, formed by the last smoothing step where that is fused
 template <typename T>
 void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
-                cudaStream_t s, int nb) {
+                cudaStream_t s, int nb, const DotOut *rho = nullptr) {
   if (l == c.L - 1) {
     launch_coarse_gemv<T>(c.nc, c.Ainv, b, x, s, nb);
+    if (rho) launch_rho_dot<T>(c, 3 * c.lev[l].nn, b, x, s, nb);
     return;
   }
   if (l >= 1 && l == c.ps) {
@@ -195,7 +198,7 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
     if constexpr (std::is_same<T, float>::value) tensor = l == 1 && l1_tensor(c);
     auto fused = [&](int in, int out) {
       if (fine_fused) {
-        launch_apply_fused<T>(c, E, in, out, a, s, nb);
+        launch_apply_fused<T>(c, E, in, out, a, s, nb, out == OUT_POST1 ? rho : nullptr);
       } else if (tensor) {
         if constexpr (std::is_same<T, float>::value) launch_l1tc(c, in, out, a, s);
       } else {
@@ -224,12 +227,12 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
   }
   // pre-smoothing from a zero guess
   launch_cheb_init<T>(n, w.dinv, b, w.r, w.d, x, ch.inv_theta, true, s, nb);
-  double rho = ch.rho0;
+  double cr = ch.rho0;   // Chebyshev recurrence coefficient
   for (int k = 1; k < o.cheb_degree; ++k) {
     level_apply<T>(c, l, w.d, nullptr, w.a, s, nb);
-    const double rn = 1.0 / (2.0 * ch.sigma - rho);
-    launch_cheb_step<T>(n, w.dinv, w.a, w.r, w.d, x, rn * rho, 2.0 * rn / ch.delta, s, nb);
-    rho = rn;
+    const double rn = 1.0 / (2.0 * ch.sigma - cr);
+    launch_cheb_step<T>(n, w.dinv, w.a, w.r, w.d, x, rn * cr, 2.0 * rn / ch.delta, s, nb);
+    cr = rn;
   }
   // residual, restriction, coarse correction, prolongation
   level_apply<T>(c, l, x, b, w.a, s, nb);
@@ -241,13 +244,14 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
   // post-smoothing from the corrected x
   level_apply<T>(c, l, x, b, w.r, s, nb);
   launch_cheb_init<T>(n, w.dinv, b, w.r, w.d, x, ch.inv_theta, false, s, nb);
-  rho = ch.rho0;
+  cr = ch.rho0;
   for (int k = 1; k < o.cheb_degree; ++k) {
     level_apply<T>(c, l, w.d, nullptr, w.a, s, nb);
-    const double rn = 1.0 / (2.0 * ch.sigma - rho);
-    launch_cheb_step<T>(n, w.dinv, w.a, w.r, w.d, x, rn * rho, 2.0 * rn / ch.delta, s, nb);
-    rho = rn;
+    const double rn = 1.0 / (2.0 * ch.sigma - cr);
+    launch_cheb_step<T>(n, w.dinv, w.a, w.r, w.d, x, rn * cr, 2.0 * rn / ch.delta, s, nb);
+    cr = rn;
   }
+  if (rho) launch_rho_dot<T>(c, n, b, x, s, nb);
 }
 
 // one CG iteration (p = z + beta p after the first): V-cycle, rho, p, q,
@@ -257,11 +261,14 @@ template <typename T>
 void cg_body(Ctx &c, int64_t n, T *x, T *r, T *z, T *p, T *q,
              const tpo_solve_opts &o, bool first, cudaStream_t s, int nb) {
   double *sc = c.scal;
-  vcycle_rec<T>(c, 0, r, z, o, s, nb);
-  launch_rho_dot<T>(c, n, r, z, s, nb);
+  // rho = r.z into slot 0, the previous one into slot 1; a frozen column
+  // (slot 6) keeps both, so a resumed recurrence finds the rho of its last
+  // active iteration
+  const DotOut rho{sc + 0, sc + 1, sc + 6};
+  vcycle_rec<T>(c, 0, r, z, o, s, nb, &rho);
   launch_cg_p<T>(n, z, p, sc, first, s, nb);
-  launch_apply_fine<T>(c, fineE(c, (T *)nullptr), p, nullptr, q, s, nb);
-  launch_dot<T>(c, n, p, q, sc + 2, nullptr, s, nb);
+  const DotOut pq{sc + 2};
+  launch_apply_fine<T>(c, fineE(c, (T *)nullptr), p, nullptr, q, s, nb, &pq);
   launch_cg_update<T>(c, n, x, r, p, q, sc, sc + 3, s, nb);
 }
 
@@ -828,8 +835,8 @@ int solve(Ctx &c, const tpo_solve_opts &o, const double *b, double *x,
   int its[kMaxBatch], st[kMaxBatch];
 
   launch_dot<double>(c, n, b, b, sc + 4, nullptr, s, nb);
-  launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb);
-  launch_dot<double>(c, n, c.r64, c.r64, sc + 5, nullptr, s, nb);
+  const DotOut rr{sc + 5};
+  launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb, &rr);
   CK(cudaGetLastError());
   if (int rc = readback(c, nb)) return rc;
   int active = 0;
@@ -860,8 +867,7 @@ int solve(Ctx &c, const tpo_solve_opts &o, const double *b, double *x,
     pcg_loop<double>(c, o, x, c.r64, c.z64, c.p64, c.q64, tgt2, o.maxit, nb,
                      frozen, its, st);
     // report the true residual
-    launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb);
-    launch_dot<double>(c, n, c.r64, c.r64, sc + 5, nullptr, s, nb);
+    launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb, &rr);
     if (int rc = readback(c, nb)) return rc;
     for (int j = 0; j < nb; ++j) {
       if (status[j] == TPO_OK) continue;   // converged before the loop
@@ -920,8 +926,7 @@ int solve(Ctx &c, const tpo_solve_opts &o, const double *b, double *x,
       // have a zero x32 and keep their x)
       launch_axpy_f32(n, x, c.x32, sc + 5, s, nb);
       CK(cudaMemsetAsync(c.x32, 0, sizeof(float) * n * nb, s));
-      launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb);
-      launch_dot<double>(c, n, c.r64, c.r64, sc + 5, nullptr, s, nb);
+      launch_apply_fine<double>(c, c.E64, x, b, c.r64, s, nb, &rr);
       launch_to_f32_scaled(n, c.r64, sc + 5, c.r32, s, nb);
       if (int rc = readback(c, nb)) return rc;
       double f[kMaxBatch], rho[kMaxBatch];

@@ -224,6 +224,7 @@ struct Ctx {
   double *scal = nullptr;   // device scalars
   double *scal_h = nullptr; // pinned host mirror
   double *part = nullptr;   // reduction partials
+  double *apply_part = nullptr;   // those of the fine operator's epilogue
   unsigned int *ticket = nullptr;
   unsigned int *gbar = nullptr;  // grid-barrier counter of the persistent
                                  // coarse-grid kernel (kernels_coarse.cu)
@@ -271,7 +272,7 @@ inline void count_launch(long long n = 1) {
   g_launches.fetch_add(n, std::memory_order_relaxed);
 }
 
-constexpr int kRedBlocks = 592;   // 4 x 148 SMs: fixed grid for reductions
+constexpr int kRedBlocks = 592;   // 4 x 148 SMs: grid of the long reductions
 
 // Right-hand sides are processed in blocks of up to kMaxBatch columns:
 // column j of a block vector lives at offset j * (3 * nn_level).  Each
@@ -302,20 +303,38 @@ constexpr int SC_LOOP_MAXIT = SC_LOOP_K + 1;
 constexpr int kScalCount = SC_LOOP_MAXIT + 1;
 constexpr int kSlotFault = 7;
 
-// fixed reduction grid (blocks per column) for a block of nb columns
-inline int red_grid(int nb) {
-  return nb <= 1 ? kRedBlocks : (kRedBlocks / nb < 148 ? 148 : kRedBlocks / nb);
+// reduction grid (blocks per column) for nb columns of length n: about one
+// 16-byte load a thread as far as that fills the chip (a thread's loads wait
+// for one another: with four of them the update of 92,000 unknowns took 8.9 us
+// for 6.4)
+inline int red_grid(int64_t n, int nb) {
+  const int full = nb <= 1 ? kRedBlocks : (kRedBlocks / nb < 148 ? 148 : kRedBlocks / nb);
+  const int64_t need = (n + 511) / 512;
+  return (int)(need < 1 ? 1 : need < full ? need : full);
 }
-// reduction scratch: red_grid(nb) * nb <= kAuxPart partials on the main
+// reduction scratch: red_grid(n, nb) * nb <= kAuxPart partials on the main
 // stream; set-up side stream i uses part + kAuxPart + i * kRedBlocks and
 // ticket + kMaxBatch + i
 constexpr int kAuxPart = 2048;
 constexpr int kPartCount = kAuxPart + kAuxStreams * kRedBlocks;
 
-// fine matrix-free operator: y = M K M u + (1-M) u, or y = b - (that)
+// A dot product formed in the epilogue of the fine-level operator, per
+// column j into out[j * kColScal] (its previous value into shift, where
+// set); a column whose skip flag is set keeps both.
+struct DotOut {
+  double *out, *shift;
+  const double *skip;
+  double *part;           // set by the launcher
+  unsigned int *ticket;
+};
+
+// fine matrix-free operator: y = M K M u + (1-M) u, or y = b - (that); dot:
+// with u.y, or with y.y
 template <typename T>
 void launch_apply_fine(const Ctx &c, const T *E, const T *u, const T *b, T *y,
-                       cudaStream_t s, int nb = 1);
+                       cudaStream_t s, int nb = 1, const DotOut *dot = nullptr);
+// partials that a dot product of the above needs for any number of columns
+int64_t apply_dot_parts(const int *nel, int sms);
 
 // fused fine-level variants: how the input is formed and what the epilogue
 // writes (sym_out_v, fused_out.cuh)
@@ -332,9 +351,11 @@ struct ApplyArgs {
   int nchunk;    // z chunks per column, set by the launcher
 };
 
+// dot (OUT_POST1 only): with b.y
 template <typename T>
 void launch_apply_fused(const Ctx &c, const T *E, int in, int out,
-                        const ApplyArgs<T> &args, cudaStream_t s, int nb = 1);
+                        const ApplyArgs<T> &args, cudaStream_t s, int nb = 1,
+                        const DotOut *dot = nullptr);
 void launch_fine_diag(const Ctx &c, double *dinv64, float *dinv32,
                       cudaStream_t s);
 void launch_fine_stencil(const Ctx &c, double *S, cudaStream_t s);
