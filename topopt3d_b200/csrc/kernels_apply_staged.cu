@@ -38,6 +38,7 @@
 // complete, and nodes of plane p-2 are written.
 #include "fused_out.cuh"
 #include "modal.cuh"
+#include "pdl.cuh"
 #include "reduce.cuh"
 
 namespace tpo {
@@ -449,6 +450,8 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     sc.put(rb + ty + 1, tx, gs, gd);
   };
 
+  pdl_wait();
+  pdl_launch_dependents();
   fetch(zs - 1);
   // two steps per trip with the state arrays swapping roles, so nothing is
   // copied between planes
@@ -559,11 +562,11 @@ void launch_mode(const Ctx &c, const T *E, const ApplyArgs<T> &args_in,
   constexpr size_t smem = staged_smem<T, IN, OUT, DOT>();
   count_launch();
   if (nb == 1)
-    k_apply_staged<T, kTY, IN, OUT, false, DOT><<<grid, dim3(32, kTY), smem, s>>>(
-        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
+    launch_pdl(k_apply_staged<T, kTY, IN, OUT, false, DOT>, grid, dim3(32, kTY), smem, s, c.nel[0],
+               c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
   else
-    k_apply_staged<T, kTY, IN, OUT, true, DOT><<<grid, dim3(32, kTY), smem, s>>>(
-        c.nel[0], c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
+    launch_pdl(k_apply_staged<T, kTY, IN, OUT, true, DOT>, grid, dim3(32, kTY), smem, s, c.nel[0],
+               c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
 }
 
 }  // namespace

@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "fused_out.cuh"
+#include "pdl.cuh"
 #include "tpo_internal.h"
 #include "umma.cuh"
 
@@ -151,16 +152,6 @@ __global__ void k_l1_corr(int cx, int cy, int cz, int64_t cap_rows, const double
     float *row = C + f * kCorrRow + nb * 9;
     for (int q = 0; q < 9; ++q) row[q] = static_cast<float>(acc[q]);
   }
-}
-
-// programmatic dependent launch: let the next kernel in the stream start,
-// and wait for the grids this one depends on (no-ops without the launch
-// attribute)
-__device__ __forceinline__ void pdl_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // cval[3 n + r] = (C u)_r on the correction rows, one warp per row; u in the

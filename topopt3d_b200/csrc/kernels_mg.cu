@@ -17,6 +17,7 @@
 
 #include "tpo_internal.h"
 #include "fused_out.cuh"
+#include "pdl.cuh"
 
 namespace tpo {
 
@@ -658,6 +659,8 @@ __global__ void __launch_bounds__(128)
   tap_weights(ix, fx, wx);
   tap_weights(iy, fy, wy);
   tap_weights(iz, fz, wz);
+  pdl_wait();
+  pdl_launch_dependents();
   const bool first = lane == 0 && ix > 0;   // loads its own left neighbour
   T s[3] = {T(0), T(0), T(0)};
   const int dl = ix > 0 ? -3 : 0, d1 = 2 * ix + 1 < fx ? 3 : 0;
@@ -720,6 +723,8 @@ __global__ void __launch_bounds__(128)
   // one or two coarse rows in y and in z
   const bool ty = (gy & 1) && gy + 1 < fy, tz = (gz & 1) && gz + 1 < fz;
   const T wyz = (ty ? T(0.5) : T(1)) * (tz ? T(0.5) : T(1));
+  pdl_wait();
+  pdl_launch_dependents();
   const int o00 = (((gz >> 1) * cy + (gy >> 1)) * cx + ix) * sn;
   const int dy = cx * sn, dz = cx * cy * sn, dr = ix + 1 < cx ? sn : 0;
   const bool last = lane == 31;   // loads its own right neighbour
@@ -797,6 +802,8 @@ __global__ void k_coarse_gemv(int64_t n, const double *__restrict__ A,
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  pdl_wait();
+  pdl_launch_dependents();
   for (int64_t row = warp; row < n; row += nwarps) {
     const double s = gemv_row(A + row * n, b, n, lane);
     if (lane == 0) x[row] = static_cast<T>(s);
@@ -1017,10 +1024,11 @@ void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *bc,
   const int *f = fine.dims, *c = coarse.dims;
   const dim3 g((unsigned)((coarse.nn + 127) / 128), 1, nb);
   if (comp)
-    k_restrict<T, true><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], rf, bc, *comp);
+    launch_pdl(k_restrict<T, true>, g, 128, 0, s, f[0], f[1], f[2], c[0], c[1], c[2], rf, bc,
+               *comp);
   else
-    k_restrict<T, false><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], rf, bc,
-                                           CompLevel<T>{});
+    launch_pdl(k_restrict<T, false>, g, 128, 0, s, f[0], f[1], f[2], c[0], c[1], c[2], rf, bc,
+               CompLevel<T>{});
 }
 template void launch_restrict<double>(const Level &, const Level &, const double *, double *,
                                       const CompLevel<double> *, cudaStream_t, int);
@@ -1034,9 +1042,9 @@ void launch_prolong_add(const Level &fine, const Level &coarse, const T *xc, T *
   const int *f = fine.dims, *c = coarse.dims;
   const dim3 g((unsigned)(((int64_t)c[0] * f[1] * f[2] + 127) / 128), 1, nb);
   if (comp)
-    k_prolong_add<T, true><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
+    launch_pdl(k_prolong_add<T, true>, g, 128, 0, s, f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
   else
-    k_prolong_add<T, false><<<g, 128, 0, s>>>(f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
+    launch_pdl(k_prolong_add<T, false>, g, 128, 0, s, f[0], f[1], f[2], c[0], c[1], c[2], xc, xf);
 }
 template void launch_prolong_add<double>(const Level &, const Level &, const double *, double *,
                                          bool, cudaStream_t, int);
@@ -1052,8 +1060,7 @@ void launch_coarse_gemv(int64_t n, const double *Ainv, const T *b, T *x,
   if (blocks > 148 * 8) blocks = 148 * 8;
   for (int col = 0; col < nb; ++col) {
     count_launch();
-    k_coarse_gemv<T><<<(int)blocks, threads, 0, s>>>(n, Ainv, b + col * n,
-                                                     x + col * n);
+    launch_pdl(k_coarse_gemv<T>, (int)blocks, threads, 0, s, n, Ainv, b + col * n, x + col * n);
   }
 }
 template void launch_coarse_gemv<double>(int64_t, const double *,

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "reduce.cuh"
 #include "tpo_internal.h"
 
@@ -98,6 +99,8 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
                        const double *__restrict__ scal, bool first) {
   using VT = Vec16<T>;
   using V = typename VT::V;
+  pdl_wait();
+  pdl_launch_dependents();
   const int j = blockIdx.y;
   const double *sc = scal + j * kColScal;
   if (sc[6] != 0.0) return;
@@ -135,6 +138,8 @@ __global__ void __launch_bounds__(kRedThreads)
                 unsigned int *ticket, double *rr) {
   using VT = Vec16<T>;
   using V = typename VT::V;
+  pdl_wait();
+  pdl_launch_dependents();
   const int j = blockIdx.y;
   const double *sc = scal + j * kColScal;
   const bool frozen = sc[6] != 0.0;
@@ -286,7 +291,7 @@ template <typename T>
 void launch_cg_p(int64_t n, const T *z, T *p, const double *scal, bool first,
                  cudaStream_t s, int nb) {
   count_launch();
-  k_cg_p<T><<<col_grid(n, nb), 256, 0, s>>>(n, z, p, scal, first);
+  launch_pdl(k_cg_p<T>, col_grid(n, nb), 256, 0, s, n, z, p, scal, first);
 }
 template void launch_cg_p<double>(int64_t, const double *, double *,
                                   const double *, bool, cudaStream_t, int);
@@ -298,8 +303,8 @@ void launch_cg_update(const Ctx &c, int64_t n, T *x, T *r, const T *p,
                       const T *q, const double *scal, double *rr,
                       cudaStream_t s, int nb) {
   count_launch();
-  k_cg_update<T><<<dim3(red_grid(n, nb), nb), kRedThreads, 0, s>>>(
-      n, x, r, p, q, scal, c.part, c.ticket, rr);
+  launch_pdl(k_cg_update<T>, dim3(red_grid(n, nb), nb), kRedThreads, 0, s, n, x, r, p, q, scal,
+             c.part, c.ticket, rr);
 }
 template void launch_cg_update<double>(const Ctx &, int64_t, double *,
                                        double *, const double *,
