@@ -530,8 +530,8 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
   const int slots = slots_cache[dev], sms = sms_cache[dev], tiles = gx * gy * nb;
   double best = 0;
   int chunks = 1;
-  // beyond four waves more chunks only add planes
-  for (int ch = 1; ch <= Nz && (ch == 1 || (int64_t)ch * tiles <= 4 * (int64_t)slots); ++ch) {
+  // beyond eight waves more chunks only add planes
+  for (int ch = 1; ch <= Nz && (ch == 1 || (int64_t)ch * tiles <= 8 * (int64_t)slots); ++ch) {
     const int zc = (Nz + ch - 1) / ch;
     const int64_t n = (int64_t)tiles * ((Nz + zc - 1) / zc), rest = n % slots;
     const double shared = slots > sms ? 1.55 : 1.0;
@@ -571,12 +571,12 @@ void launch_mode(const Ctx &c, const T *E, const ApplyArgs<T> &args_in,
 
 }  // namespace
 
-// staged_grid makes at most max(4 x resident CTAs, tiles x columns) CTAs
+// staged_grid makes at most max(8 x resident CTAs, tiles x columns) CTAs
 int64_t apply_dot_parts(const int *nel, int sms) {
   const int64_t gx = (nel[0] + 1 + kLanesOut - 1) / kLanesOut;
   const int64_t gy = (nel[1] + 1 + kTY - 2) / (kTY - 1);
   constexpr int kMaxPerSm = 2048 / (32 * kTY);
-  return std::max<int64_t>(4 * kMaxPerSm * (int64_t)sms, gx * gy * kMaxBatch);
+  return std::max<int64_t>(8 * kMaxPerSm * (int64_t)sms, gx * gy * kMaxBatch);
 }
 
 template <typename T>
