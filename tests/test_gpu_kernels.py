@@ -182,3 +182,34 @@ def test_cg_dot_products(T, nel, levels, degree, nb):
         alone.append(t.solve(b[j].copy(), Uj, opts=o)["iterations"])
         assert np.linalg.norm(Uj - U[j]) <= 1e-5 * np.linalg.norm(Uj)
     assert its == sum(alone)
+
+
+# the captured CG loop outlives the operator: one column and a block, both
+# forms, with other smoother options and other boundary conditions in between
+@pytest.mark.parametrize("nb", [1, 3])
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("nel", [(12, 6, 6), (32, 16, 16)])
+def test_a_new_operator_solves_as_in_a_new_context(T, nel, mixed, nb):
+    """After other designs, options and supports the context solves as one that
+    has seen the last of them only, bit for bit."""
+    prec = T.PREC_MIXED if mixed else T.PREC_FP64
+    b = np.random.default_rng(4).standard_normal((nb, 3 * int(np.prod(np.add(nel, 1)))))
+
+    def step(t, bc, seed, degree):
+        o = T.default_opts(precision=prec, cheb_degree=degree)
+        t.set_bc_arrays(np.zeros(t.nNode, np.uint8), np.zeros(3 * t.nNode))
+        P.apply_bcs(t, bc)
+        t.FEInitialize()
+        t.MatIntFnc(np.random.default_rng(seed).uniform(0.3, 0.8, t.nElem))
+        t.FEAssemble(o)
+        t.set("U", np.zeros(3 * t.nNode))
+        t.FESolve(o)
+        U = np.zeros_like(b)
+        t.solve(b, U, nrhs=nb, opts=o)
+        return np.array(t.U), U
+    one, two = P.cantilever_bcs(nel), P.bcs("cfg2", nel)
+    t = T.TopOpt(nel, mg_levels=3)
+    for bc, seed, degree in ((one, 1, 2), (one, 2, 2), (one, 2, 1), (two, 3, 2), (one, 4, 2)):
+        got = step(t, bc, seed, degree)
+        ref = step(T.TopOpt(nel, mg_levels=3), bc, seed, degree)
+        assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])

@@ -24,7 +24,7 @@ struct CoarseLevel {
   // the Galerkin stencil by CTA: block nb, entry rs of node s * npc + i at
   // A[(s * 243 + nb * 9 + rs) * npcp + i]
   const T *A;
-  const T *dinv;   // 1 / diag, 3 n + c
+  const T *dinv;   // 1 / (lambda diag), 3 n + c
   T *b;            // right-hand side (restricted residual of the parent)
   T *xpre;         // pre-smoothed iterate, then + P x_child
   T *xout;         // post-smoothed result (read by the parent)

@@ -207,6 +207,17 @@ __global__ void k_power_start(int64_t n, T *a) {
     a[i] = static_cast<T>(start_value((uint64_t)i));
 }
 
+__global__ void k_scale_dinv(int64_t n, const double *nrm2, const double *prev2,
+                             double *dinv64, float *dinv32) {
+  const double lam = sqrt(*nrm2 / *prev2);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double d = dinv64[i] / lam;
+    dinv64[i] = d;
+    dinv32[i] = static_cast<float>(d);
+  }
+}
+
 // b = float(a / sqrt(*nrm2)) per column (a zero column stays zero)
 __global__ void k_to_f32_scaled(int64_t n, const double *a, const double *nrm2,
                                 float *b) {
@@ -322,6 +333,12 @@ void launch_power_start(int64_t n, T *a, cudaStream_t s) {
 }
 template void launch_power_start<double>(int64_t, double *, cudaStream_t);
 template void launch_power_start<float>(int64_t, float *, cudaStream_t);
+
+void launch_scale_dinv(int64_t n, const double *nrm2, const double *prev2, double *dinv64,
+                       float *dinv32, cudaStream_t s) {
+  count_launch();
+  k_scale_dinv<<<grid_for(n, 256), 256, 0, s>>>(n, nrm2, prev2, dinv64, dinv32);
+}
 
 void launch_to_f32_scaled(int64_t n, const double *a, const double *scal,
                           float *b, cudaStream_t s, int nb) {

@@ -23,12 +23,15 @@ double now_ms() {
       .count();
 }
 
+// Chebyshev coefficients on [cheb_lo, cheb_hi] x lambda.  The smoothers work
+// with (lambda D)^-1 (launch_scale_dinv), so the coefficients depend on the
+// options alone, and the loop graphs stay valid when K changes.
 struct Cheb {
   double inv_theta, sigma, delta, rho0, theta;
 };
 
-Cheb cheb_of(double lam, const tpo_solve_opts &o) {
-  const double a = o.cheb_lo * lam, b = o.cheb_hi * lam;
+Cheb cheb_of(const tpo_solve_opts &o) {
+  const double a = o.cheb_lo, b = o.cheb_hi;
   const double theta = 0.5 * (b + a), delta = 0.5 * (b - a);
   const double sigma = theta / delta;
   return {1.0 / theta, sigma, delta, 1.0 / sigma, theta};
@@ -110,7 +113,7 @@ CoarseCycle<T> coarse_cycle_params(Ctx &c, const tpo_solve_opts &o) {
       L.xpre = reinterpret_cast<T *>(v.w32);
       L.d1 = reinterpret_cast<T *>(v.e32);
     }
-    const Cheb ch = cheb_of(v.lam, o);
+    const Cheb ch = cheb_of(o);
     L.inv_theta = static_cast<T>(ch.inv_theta);
     L.deg = std::min(o.cheb_degree, kMaxChebDegree);
     double rho = ch.rho0;
@@ -142,7 +145,7 @@ void restrict_to(Ctx &c, int l, const T *r, const tpo_solve_opts &o, cudaStream_
   Level &v = c.lev[l], &cv = c.lev[l + 1];
   LV<T> cw = lv(cv, (T *)nullptr);
   if (comp_level(c, l + 1)) {
-    const CompLevel<T> top{cw.dinv, cw.d, static_cast<T>(cheb_of(cv.lam, o).inv_theta)};
+    const CompLevel<T> top{cw.dinv, cw.d, static_cast<T>(cheb_of(o).inv_theta)};
     launch_restrict<T>(v, cv, r, cw.b, &top, s, nb);
   } else {
     launch_restrict<T>(v, cv, r, cw.b, nullptr, s, nb);
@@ -176,7 +179,7 @@ void vcycle_rec(Ctx &c, int l, const T *b, T *x, const tpo_solve_opts &o,
   Level &v = c.lev[l];
   LV<T> w = lv(v, (T *)nullptr);
   const int64_t n = 3 * v.nn;
-  const Cheb ch = cheb_of(v.lam, o);
+  const Cheb ch = cheb_of(o);
   const bool fine_fused = (l == 0);
   const bool sym_fused = (l >= 1 && l < c.ps && nb == 1);
   if (o.cheb_degree == 2 && (fine_fused || sym_fused)) {
@@ -424,8 +427,7 @@ int pcg_loop(Ctx &c, const tpo_solve_opts &o, T *x, T *r, T *z, T *p, T *q,
   cudaStream_t s = c.stream;
   const int64_t n = 3 * c.nn;
   cudaGraphExec_t &g = (sizeof(T) == 8) ? c.graph64 : c.graph32;
-  const void *&gx = (sizeof(T) == 8) ? c.graph64_x : c.graph32_x;
-  int &gnb = (sizeof(T) == 8) ? c.graph64_nb : c.graph32_nb;
+  LoopKey &gkey = (sizeof(T) == 8) ? c.graph64_key : c.graph32_key;
   long long &gnodes = (sizeof(T) == 8) ? c.graph64_nodes : c.graph32_nodes;
   int active = 0;
   for (int j = 0; j < nb; ++j) {
@@ -486,7 +488,8 @@ int pcg_loop(Ctx &c, const tpo_solve_opts &o, T *x, T *r, T *z, T *p, T *q,
       if (int rc = host_test(k)) return rc;
     }
     if (active && k < maxit) {
-      if (!g || gx != (const void *)x || gnb != nb) {
+      const LoopKey key{x, c.l1_C, o.cheb_lo, o.cheb_hi, o.cheb_degree, nb, c.l1_nrows};
+      if (!g || !(gkey == key)) {
         if (g) {
           cudaGraphExecDestroy(g);
           g = nullptr;
@@ -512,8 +515,7 @@ int pcg_loop(Ctx &c, const tpo_solve_opts &o, T *x, T *r, T *z, T *p, T *q,
           goto done;
         }
         CK(c.coarse_err);
-        gx = x;
-        gnb = nb;
+        gkey = key;
       }
       // loop state: per column target, iterations so far and status; the
       // iterations done and the limit (one copy from the pinned mirror; the
@@ -569,8 +571,7 @@ void invalidate_graphs(Ctx &c) {
   if (c.graph64) cudaGraphExecDestroy(c.graph64);
   if (c.graph32) cudaGraphExecDestroy(c.graph32);
   c.graph64 = c.graph32 = nullptr;
-  c.graph64_x = c.graph32_x = nullptr;
-  c.graph64_nb = c.graph32_nb = 0;
+  c.graph64_key = c.graph32_key = LoopKey{};
 }
 
 // w = D^-1 A_l a, in the operator kernels' epilogue
@@ -597,7 +598,8 @@ void level_scaled_apply(Ctx &c, int l, const T *a, T *w, cudaStream_t s) {
   }
 }
 
-// power iteration for lambda_max(D^-1 A_l) on stream s, no host sync.  The
+// power iteration for lambda_max(D^-1 A_l) on stream s, no host sync (dinv is
+// D^-1 then; launch_scale_dinv turns it into (lambda D)^-1 afterwards).  The
 // start vector is the splitmix64 sequence the oracle shares.  The iterates
 // v_{k+1} = D^-1 A v_k are not normalised (lambda_max(D^-1 A) is a small
 // number, so 15 steps stay far inside the FP64 range), so a step is one
@@ -640,24 +642,18 @@ double power_lambda(const Ctx &c, int l) {
   return std::sqrt(c.scal_h[SC_POWER + l] / c.scal_h[SC_POWER_PREV + l]);
 }
 
-int estimate_lambda(Ctx &c, int l, int its, double *lam) {
-  cudaStream_t s = c.stream;
-  power_iteration(c, l, its, s, nullptr, nullptr, false);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(c.scal_h + SC_POWER, c.scal + SC_POWER,
-                     sizeof(double) * (SC_POWER_PREV + kMaxLevels - SC_POWER),
-                     cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  *lam = power_lambda(c, l);
-  return TPO_OK;
-}
-
 namespace {
 
 // the hierarchy on stream s (see setup_hierarchy)
 int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
   const double t0 = now_ms();
-  invalidate_graphs(c);
+  // the loop graphs hold pointers and option values only (LoopKey): those on
+  // the context's own vectors outlive the operator.  Building one takes 0.23
+  // ms, a fifth of a step of 12x6x6 when it was done after each assembly.
+  if (c.graph64 && c.graph64_key.x != c.U) {
+    cudaGraphExecDestroy(c.graph64);
+    c.graph64 = nullptr;
+  }
   // Chebyshev bounds (power iterations) of each smoothed level run on a
   // side stream as soon as that level's operator is built on s, with their
   // own reduction scratch: level l on side stream l % kAuxStreams, so the
@@ -674,6 +670,8 @@ int setup_on(Ctx &c, const tpo_solve_opts &o, cudaStream_t s) {
     power_iteration(c, l, o.power_its, c.aux_stream[i],
                     c.part + kAuxPart + i * kRedBlocks, c.ticket + kMaxBatch + i,
                     o.precision == TPO_PREC_MIXED);
+    launch_scale_dinv(3 * c.lev[l].nn, c.scal + SC_POWER + l, c.scal + SC_POWER_PREV + l,
+                      c.lev[l].dinv64, c.lev[l].dinv32, c.aux_stream[i]);
     return TPO_OK;
   };
   auto join = [&]() {

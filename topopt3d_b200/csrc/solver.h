@@ -6,7 +6,6 @@
 namespace tpo {
 
 void invalidate_graphs(Ctx &c);
-int estimate_lambda(Ctx &c, int level, int its, double *lam);
 int setup_hierarchy(Ctx &c, const tpo_solve_opts &o);
 int vcycle_apply(Ctx &c, const tpo_solve_opts &o, int precision,
                  const double *r, double *z);

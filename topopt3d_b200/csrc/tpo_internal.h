@@ -81,7 +81,7 @@ struct Level {
   // 3r + s) * nn + n]; H32 a copy by tiles (kernels_mg.cu)
   double *H64 = nullptr;
   float *H32 = nullptr;
-  double *dinv64 = nullptr;
+  double *dinv64 = nullptr;   // (lambda_max D)^-1 once set up
   float *dinv32 = nullptr;
   double lam = 0.0;
   // V-cycle work vectors (3*nn per column, Ctx::nb_cap columns); e = second
@@ -113,6 +113,19 @@ struct CoarseInvPlan {
 constexpr int kAuxStreams = 4;
 // GMG levels of one context
 constexpr int kMaxLevels = 16;
+
+// what a loop graph of CG (solver.cu) has of its launches' arguments that can
+// change: the solution vector, the level-1 correction rows, the smoother's
+// options, the columns
+struct LoopKey {
+  const void *x = nullptr, *l1 = nullptr;
+  double cheb_lo = 0, cheb_hi = 0;
+  int cheb_degree = 0, nb = 0, l1_rows = 0;
+  bool operator==(const LoopKey &k) const {
+    return x == k.x && l1 == k.l1 && cheb_lo == k.cheb_lo && cheb_hi == k.cheb_hi &&
+           cheb_degree == k.cheb_degree && nb == k.nb && l1_rows == k.l1_rows;
+  }
+};
 
 struct Ctx {
   tpo_mesh_params prm{};
@@ -259,8 +272,7 @@ struct Ctx {
   // CUDA graphs of the CG iteration loop (a device-side while loop around
   // the iteration body), keyed on (x, columns)
   cudaGraphExec_t graph64 = nullptr, graph32 = nullptr;
-  const void *graph64_x = nullptr, *graph32_x = nullptr;
-  int graph64_nb = 0, graph32_nb = 0;
+  LoopKey graph64_key, graph32_key;
   long long graph64_nodes = 0, graph32_nodes = 0;
 };
 
@@ -457,6 +469,9 @@ void launch_dot(const Ctx &c, int64_t n, const T *a, const T *b, double *out,
 template <typename T>
 void launch_rho_dot(const Ctx &c, int64_t n, const T *r, const T *z, cudaStream_t s,
                     int nb);
+// dinv = (lambda D)^-1 from D^-1, lambda = sqrt(*nrm2 / *prev2), both copies
+void launch_scale_dinv(int64_t n, const double *nrm2, const double *prev2, double *dinv64,
+                       float *dinv32, cudaStream_t s);
 template <typename T>
 void launch_cg_p(int64_t n, const T *z, T *p, const double *scal, bool first,
                  cudaStream_t s, int nb = 1);
