@@ -660,7 +660,6 @@ __global__ void __launch_bounds__(128)
   tap_weights(iy, fy, wy);
   tap_weights(iz, fz, wz);
   pdl_wait();
-  pdl_launch_dependents();
   const bool first = lane == 0 && ix > 0;   // loads its own left neighbour
   T s[3] = {T(0), T(0), T(0)};
   const int dl = ix > 0 ? -3 : 0, d1 = 2 * ix + 1 < fx ? 3 : 0;
@@ -690,6 +689,7 @@ __global__ void __launch_bounds__(128)
       }
     }
   }
+  pdl_launch_dependents();
   if (t >= nnc) return;
   T *o = bc + col * 3 * (int64_t)nnc;
 #pragma unroll

@@ -100,7 +100,6 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
   using VT = Vec16<T>;
   using V = typename VT::V;
   pdl_wait();
-  pdl_launch_dependents();
   const int j = blockIdx.y;
   const double *sc = scal + j * kColScal;
   if (sc[6] != 0.0) return;
@@ -126,6 +125,7 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
     tail = nv * VT::W;
   }
   for (int64_t i = tail + t0; i < n; i += st) p[i] = first ? z[i] : z[i] + beta * p[i];
+  pdl_launch_dependents();
 }
 
 // x += alpha p ; r -= alpha q ; rr = r.r   with alpha = rho / (p.q), per
@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(kRedThreads)
   using VT = Vec16<T>;
   using V = typename VT::V;
   pdl_wait();
-  pdl_launch_dependents();
   const int j = blockIdx.y;
   const double *sc = scal + j * kColScal;
   const bool frozen = sc[6] != 0.0;
@@ -186,6 +185,7 @@ __global__ void __launch_bounds__(kRedThreads)
     }
     s += static_cast<double>(ri) * static_cast<double>(ri);
   }
+  pdl_launch_dependents();
   finish_reduction(s, threadIdx.x, blockDim.x, blockIdx.x, gridDim.x, part + j * gridDim.x,
                    ticket + j, rr + j * kColScal,
                    nullptr);
