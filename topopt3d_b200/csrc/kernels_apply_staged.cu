@@ -483,14 +483,16 @@ constexpr size_t staged_smem() {
   return (kTY + 1) * (4 * Six<T>::bytes_per_row() + Staged<IN, OUT, DOT>::planes() * 96 * sizeof(T));
 }
 
-template <typename T, int IN, int OUT, bool DOT = false>
-void set_smem_attr() {
-  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, false, DOT>,
+// opts a kernel in to > 48 KB of dynamic shared memory (the FP64 tiles), at its
+// first launch on a device (setting it loads the kernel)
+template <typename T, int IN, int OUT, bool COLS, bool DOT>
+void set_smem_attr(int dev) {
+  static unsigned long long done = 0;   // bit per device
+  if ((done >> (dev & 63)) & 1ull) return;
+  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, COLS, DOT>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)staged_smem<T, IN, OUT, DOT>());
-  cudaFuncSetAttribute(k_apply_staged<T, kTY, IN, OUT, true, DOT>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)staged_smem<T, IN, OUT, DOT>());
+  done |= 1ull << (dev & 63);
 }
 
 // grid of the staged kernel: 30 x (kTY-1) owned node columns per CTA, and z
@@ -513,16 +515,7 @@ void staged_grid(const Ctx &c, int nb, dim3 &grid, int &zchunk) {
   static unsigned long long attr_set = 0;   // bit per device
   static int slots_cache[64] = {0}, sms_cache[64] = {0};
   if (!((attr_set >> dev) & 1ull)) {
-    // opt in to > 48 KB of dynamic shared memory (the FP64 tiles)
-    set_smem_attr<T, IN_U, OUT_Y>();
-    set_smem_attr<T, IN_U, OUT_RESID>();
-    set_smem_attr<T, IN_CHEB, OUT_CHEB2>();
-    set_smem_attr<T, IN_U, OUT_POST0>();
-    set_smem_attr<T, IN_U, OUT_POST1>();
-    set_smem_attr<T, IN_U, OUT_SCALE>();
-    set_smem_attr<T, IN_U, OUT_Y, true>();
-    set_smem_attr<T, IN_U, OUT_RESID, true>();
-    set_smem_attr<T, IN_U, OUT_POST1, true>();
+    set_smem_attr<T, IN_CHEB, OUT_CHEB2, true, false>(dev);
     int per_sm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, k_apply_staged<T, kTY, IN_CHEB, OUT_CHEB2, true, false>, 32 * kTY,
@@ -566,12 +559,15 @@ void launch_mode(const Ctx &c, const T *E, const ApplyArgs<T> &args_in,
       sizeof(T) == 8 ? (const void *)&c.kh64 : (const void *)&c.kh32);
   constexpr size_t smem = staged_smem<T, IN, OUT, DOT>();
   count_launch();
-  if (nb == 1)
+  if (nb == 1) {
+    set_smem_attr<T, IN, OUT, false, DOT>(c.device);
     launch_pdl(k_apply_staged<T, kTY, IN, OUT, false, DOT>, grid, dim3(32, kTY), smem, s, c.nel[0],
                c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
-  else
+  } else {
+    set_smem_attr<T, IN, OUT, true, DOT>(c.device);
     launch_pdl(k_apply_staged<T, kTY, IN, OUT, true, DOT>, grid, dim3(32, kTY), smem, s, c.nel[0],
                c.nel[1], c.nel[2], zchunk, E, c.idm, args, kh, dot);
+  }
 }
 
 }  // namespace
