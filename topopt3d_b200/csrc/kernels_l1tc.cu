@@ -36,6 +36,7 @@
 
 #include "fused_out.cuh"
 #include "pdl.cuh"
+#include "solver.h"
 #include "tpo_internal.h"
 #include "umma.cuh"
 
@@ -550,6 +551,7 @@ int l1tc_prepare(Ctx &c, const double *Sc, int nslots, cudaStream_t s) {
   const size_t rows = std::max<size_t>(8 * (size_t)nslots, 1);
   if (rows > c.l1_cap) {
     if (cudaStreamSynchronize(s) != cudaSuccess) return TPO_E_CUDA;
+    invalidate_graphs(c);   // they hold l1_C, l1_rows and l1_cap
     if (c.l1_C) cudaFree(c.l1_C);
     if (c.l1_rows) cudaFree(c.l1_rows);
     c.l1_C = nullptr;

@@ -488,7 +488,7 @@ int pcg_loop(Ctx &c, const tpo_solve_opts &o, T *x, T *r, T *z, T *p, T *q,
       if (int rc = host_test(k)) return rc;
     }
     if (active && k < maxit) {
-      const LoopKey key{x, c.l1_C, o.cheb_lo, o.cheb_hi, o.cheb_degree, nb, c.l1_nrows};
+      const LoopKey key{x, o.cheb_lo, o.cheb_hi, o.cheb_degree, nb, c.l1_nrows};
       if (!g || !(gkey == key)) {
         if (g) {
           cudaGraphExecDestroy(g);

@@ -115,14 +115,17 @@ constexpr int kAuxStreams = 4;
 constexpr int kMaxLevels = 16;
 
 // what a loop graph of CG (solver.cu) has of its launches' arguments that can
-// change: the solution vector, the level-1 correction rows, the smoother's
-// options, the columns
+// change: the solution vector, the number of level-1 correction rows, the
+// smoother's options, the columns.  The other pointers it holds are those of
+// the context's own buffers: whoever frees one of them (ensure_columns,
+// l1tc_prepare) drops the graphs with it (invalidate_graphs), since a later
+// buffer may have the same address.
 struct LoopKey {
-  const void *x = nullptr, *l1 = nullptr;
+  const void *x = nullptr;
   double cheb_lo = 0, cheb_hi = 0;
   int cheb_degree = 0, nb = 0, l1_rows = 0;
   bool operator==(const LoopKey &k) const {
-    return x == k.x && l1 == k.l1 && cheb_lo == k.cheb_lo && cheb_hi == k.cheb_hi &&
+    return x == k.x && cheb_lo == k.cheb_lo && cheb_hi == k.cheb_hi &&
            cheb_degree == k.cheb_degree && nb == k.nb && l1_rows == k.l1_rows;
   }
 };
