@@ -56,3 +56,25 @@ def test_more_general_elements_with_the_same_correction_rows(T):
         t.apply(u, y)
         assert np.linalg.norm(F - y) <= 1.0001e-8 * np.linalg.norm(F)
     assert abs(its - ref) <= 1
+
+
+@pytest.mark.parametrize("supports", ["face", "face and ring"])
+def test_an_assembly_does_not_depend_on_those_before(T, supports):
+    """The smoothers' bounds and the solution of a design are the same, bit for
+    bit, whether the context has assembled it before, or other supports, or
+    nothing: each correction row is one warp's sum and every reduction has a
+    fixed order."""
+    x = np.random.default_rng(4).uniform(0.3, 0.8, int(np.prod(NEL)))
+    base = P.cantilever_bcs(NEL)
+    bc = base + (RING if "ring" in supports else [])
+    other = base + ([] if "ring" in supports else RING)
+    new = T.TopOpt(NEL, mg_levels=LEVELS)
+    ref = step(T, new, bc, x)
+    lam = [new.level_lambda(l) for l in range(LEVELS - 1)]
+    again = step(T, new, bc, x)
+    t = T.TopOpt(NEL, mg_levels=LEVELS)
+    step(T, t, other, x)
+    after = step(T, t, bc, x)
+    for c, got in ((new, again), (t, after)):
+        assert [c.level_lambda(l) for l in range(LEVELS - 1)] == lam
+        assert got[1] == ref[1] and np.array_equal(got[0], ref[0])

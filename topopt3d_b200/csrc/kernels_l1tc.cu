@@ -562,6 +562,9 @@ int l1tc_prepare(Ctx &c, const double *Sc, int nslots, cudaStream_t s) {
       return TPO_E_CUDA;
     c.l1_cap = rows;
   }
+  // the launches of the set-up itself go by this bound (the set-up reads the
+  // count back at its end)
+  c.l1_nrows = nslots > 0 ? (int)rows : 0;
   int tx, ty, zc, nz;
   l1tc_grid(v, &tx, &ty, &zc, &nz);
   if (cudaMemsetAsync(c.l1_count, 0, sizeof(unsigned int), s) != cudaSuccess ||
@@ -582,11 +585,11 @@ void launch_l1tc(const Ctx &c, int in, int out, const ApplyArgs<float> &a, cudaS
   const Level &v = c.lev[1];
   int tx, ty, zc, nz;
   l1tc_grid(v, &tx, &ty, &zc, &nz);
-  // C u on the correction rows first (a warp per row; the row count is the
-  // one the last set-up read back)
+  // C u on the correction rows first, a warp per row: the kernel goes by the
+  // count on the device; the host's is that count, or a bound during a set-up
   const bool pdl = c.l1_nrows > 0;
   if (pdl) {
-    const int blocks = (c.l1_nrows + 3) / 4;
+    const int blocks = grid_for(c.l1_nrows, 4);
     count_launch();
     if (in == IN_CHEB)
       k_l1_corr_apply<IN_CHEB><<<blocks, 128, 0, s>>>(v.dims[0], v.dims[1], v.dims[2],

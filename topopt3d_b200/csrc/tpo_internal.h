@@ -219,7 +219,7 @@ struct Ctx {
   float *l1_cval = nullptr;
   uint8_t *l1_cflag = nullptr;
   unsigned int *l1_count = nullptr;
-  int l1_nrows = 0;   // host copy of the row count (read at the end of set-up)
+  int l1_nrows = 0;   // host copy of the row count (a bound until the end of set-up)
   int *l1_fault = nullptr;
   // scratch of the dimension-by-dimension Galerkin products (levels >= 1)
   double *gd_tmp = nullptr;
