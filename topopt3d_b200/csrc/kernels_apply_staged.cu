@@ -168,7 +168,7 @@ struct Six<double> {
 template <typename T, int TY, int IN, int OUT, bool COLS, bool DOT>
 __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     k_apply_staged(int nelx, int nely, int nelz, int zchunk,
-                   const T *__restrict__ E, const uint8_t *__restrict__ fix,
+                   const T *E, const uint8_t *fix,
                    const ApplyArgs<T> args_in, const Kh<T> kh, const DotOut dot) {
   const int Nx = nelx + 1, Ny = nely + 1, Nz = nelz + 1;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     if (z >= 0 && z < Nz) {
       const int n = nofs + z * NP;
       if (nin) {
-        pf = __ldg(fix + n);
+        pf = load_ro(fix + n);
         if (Sg::kIn) {
           T *db = slot_at(Sg::kSlotB, z, ty), *dd = slot_at(Sg::kSlotD, z, ty);
 #pragma unroll
@@ -250,12 +250,12 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
           }
         } else {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) pu[c] = __ldg(args.u + 3 * (int64_t)n + c);
+          for (int c = 0; c < 3; ++c) pu[c] = load_ro(args.u + 3 * (int64_t)n + c);
         }
       }
       if (nin2) {
         const int n2 = nofs2 + z * NP;
-        pf2 = __ldg(fix + n2);
+        pf2 = load_ro(fix + n2);
         if (Sg::kIn) {
           T *db = slot_at(Sg::kSlotB, z, TY), *dd = slot_at(Sg::kSlotD, z, TY);
 #pragma unroll
@@ -265,12 +265,12 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
           }
         } else {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) pq[c] = __ldg(args.u + 3 * (int64_t)n2 + c);
+          for (int c = 0; c < 3; ++c) pq[c] = load_ro(args.u + 3 * (int64_t)n2 + c);
         }
       }
     }
     const int ez = z - 1;
-    if (exy && ez >= 0 && ez < nelz) pE = __ldg(E + eofs + ez * EP);
+    if (exy && ez >= 0 && ez < nelz) pE = load_ro(E + eofs + ez * EP);
   };
   // the epilogue operands of plane z
   auto fetch_out = [&](int z) {
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
           else if (Sg::kU)
             uv = su[c];
           else if (fixed)
-            uv = __ldg(args.u + i + c);
+            uv = load_ro(args.u + i + c);
           const T yv = sym_out_v<T, OUT>(args, i + c, fixed ? uv : val[c], uv, bi, di, yi);
           if (DOT)
             dsum += static_cast<double>(OUT == OUT_Y ? uv : OUT == OUT_RESID ? yv : bi) *
@@ -451,11 +451,6 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
   };
 
   pdl_wait();
-  // the steps of a power iteration share the chip with the rest of the set-up,
-  // and the next one's blocks hold its place when they come early; in the CG
-  // iteration blocks that wait are in the way (91x47x53 mixed: 3.17 ms a solve
-  // for 3.07)
-  if (OUT == OUT_SCALE) pdl_launch_dependents();
   fetch(zs - 1);
   // two steps per trip with the state arrays swapping roles, so nothing is
   // copied between planes
@@ -463,7 +458,9 @@ __global__ void __launch_bounds__(32 * TY, sizeof(T) == 4 ? 2 : 1)
     step(p, FA, FB, CA, CB);
     if (p + 1 <= ze + 1) step(p + 1, FB, FA, CB, CA);
   }
-  if (OUT != OUT_SCALE) pdl_launch_dependents();
+  // after the stores (pdl.cuh); blocks that come earlier and wait are in the
+  // way, too (91x47x53 mixed: 3.17 ms a solve for 3.07)
+  pdl_launch_dependents();
   if (DOT) {
     // one partial per CTA of the column
     const int nchunk = args_in.nchunk, col = COLS ? (int)blockIdx.z / nchunk : 0;

@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(Tile<T>::kThreads)
 // matrix
 template <int T>
 __global__ void __launch_bounds__(Tile<T>::kThreads)
-    k_ci_fg(const int4 *__restrict__ tasks, double *W, const double *__restrict__ P, double *F,
+    k_ci_fg(const int4 *__restrict__ tasks, double *W, const double *P, double *F,
             double *G) {
   extern __shared__ __align__(16) double smem[];
   constexpr int ld = Tile<T>::kLd;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(Tile<T>::kThreads)
 template <int T>
 __global__ void __launch_bounds__(Tile<T>::kThreads)
     k_ci_update(const int4 *__restrict__ tasks, const int2 *__restrict__ pairs, double *W,
-                const double *__restrict__ F, const double *__restrict__ G, double *P,
+                const double *F, const double *G, double *P,
                 const int *__restrict__ dofs, int *info) {
   extern __shared__ __align__(16) double smem[];
   constexpr int ld = Tile<T>::kLd;
@@ -327,7 +327,7 @@ __global__ void k_ci_fill(int nx, int ny, int nz, const double *__restrict__ S,
 
 // Ainv (n x n, dof order) = -W, one CTA per tile on or below the diagonal
 __global__ void k_ci_final(int n, int T, const int *__restrict__ dofs,
-                           const double *__restrict__ W, double *__restrict__ Ainv) {
+                           const double *W, double *__restrict__ Ainv) {
   extern __shared__ __align__(16) double smem[];
   const int I = blockIdx.x, J = blockIdx.y;
   pdl_wait();

@@ -647,8 +647,8 @@ __device__ __forceinline__ void tap_weights(int c, int N, T (&w)[3]) {
 // blockIdx.z = column; a thread per coarse node
 template <typename T, bool COMP>
 __global__ void __launch_bounds__(128)
-    k_restrict(int fx, int fy, int fz, int cx, int cy, int cz, const T *__restrict__ rf,
-               T *__restrict__ bc, const CompLevel<T> comp) {
+    k_restrict(int fx, int fy, int fz, int cx, int cy, int cz, const T *rf, T *__restrict__ bc,
+               const CompLevel<T> comp) {
   const int lane = threadIdx.x & 31;
   const int nnc = cx * cy * cz, t = (int)blockIdx.x * 128 + threadIdx.x;
   const int I = min(t, nnc - 1);
@@ -673,9 +673,9 @@ __global__ void __launch_bounds__(128)
       const T *p = rf + 3 * ((z * fy + y) * fx + 2 * ix);   // 32-bit: 3 nn < 2^31
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
-        a0[b][q] = p[q];
-        a1[b][q] = p[d1 + q];
-        am[b][q] = first ? p[dl + q] : T(0);
+        a0[b][q] = load_ro(p + q);
+        a1[b][q] = load_ro(p + d1 + q);
+        am[b][q] = first ? load_ro(p + dl + q) : T(0);
       }
     }
 #pragma unroll
@@ -689,7 +689,6 @@ __global__ void __launch_bounds__(128)
       }
     }
   }
-  pdl_launch_dependents();
   if (t >= nnc) return;
   T *o = bc + col * 3 * (int64_t)nnc;
 #pragma unroll
@@ -701,6 +700,7 @@ __global__ void __launch_bounds__(128)
       o[3 * I + q] = s[q];
     }
   }
+  pdl_launch_dependents();
 }
 
 // x_f += P x_c for nb columns; COMP: x_c component by component.
@@ -708,8 +708,7 @@ __global__ void __launch_bounds__(128)
 // nodes 2 ix and 2 ix + 1
 template <typename T, bool COMP>
 __global__ void __launch_bounds__(128)
-    k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz, const T *__restrict__ xc,
-                  T *__restrict__ xf) {
+    k_prolong_add(int fx, int fy, int fz, int cx, int cy, int cz, const T *xc, T *__restrict__ xf) {
   const int lane = threadIdx.x & 31;
   const int total = cx * fy * fz, t = (int)blockIdx.x * 128 + threadIdx.x;
   const int i = min(t, total - 1);
@@ -724,7 +723,6 @@ __global__ void __launch_bounds__(128)
   const bool ty = (gy & 1) && gy + 1 < fy, tz = (gz & 1) && gz + 1 < fz;
   const T wyz = (ty ? T(0.5) : T(1)) * (tz ? T(0.5) : T(1));
   pdl_wait();
-  pdl_launch_dependents();
   const int o00 = (((gz >> 1) * cy + (gy >> 1)) * cx + ix) * sn;
   const int dy = cx * sn, dz = cx * cy * sn, dr = ix + 1 < cx ? sn : 0;
   const bool last = lane == 31;   // loads its own right neighbour
@@ -735,8 +733,8 @@ __global__ void __launch_bounds__(128)
     const T *p = xc + (o00 + ((k & 1) ? dy : 0) + ((k >> 1) ? dz : 0));
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      v[q] += p[q * sc];
-      if (last) r[q] += p[dr + q * sc];
+      v[q] += load_ro(p + q * sc);
+      if (last) r[q] += load_ro(p + dr + q * sc);
     }
   }
   // the warp's 32 x 6 corrections through shared memory, so that the fine
@@ -772,23 +770,22 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
   for (int k = 0; k < 6; ++k)
     if (at[k] >= 0) xf[at[k]] = f[k] + vals[wp][lane + 32 * k];
+  pdl_launch_dependents();
 }
 
 // one row of x = Ainv b by one warp: four independent partial sums so the
 // loads of consecutive chunks overlap; result valid in every lane
 template <typename T>
-__device__ __forceinline__ double gemv_row(const double *__restrict__ a,
-                                           const T *__restrict__ b, int64_t n,
-                                           int lane) {
+__device__ __forceinline__ double gemv_row(const double *a, const T *b, int64_t n, int lane) {
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
   int64_t k = lane;
   for (; k + 96 < n; k += 128) {
-    s0 += a[k] * static_cast<double>(b[k]);
-    s1 += a[k + 32] * static_cast<double>(b[k + 32]);
-    s2 += a[k + 64] * static_cast<double>(b[k + 64]);
-    s3 += a[k + 96] * static_cast<double>(b[k + 96]);
+    s0 += load_ro(a + k) * static_cast<double>(load_ro(b + k));
+    s1 += load_ro(a + k + 32) * static_cast<double>(load_ro(b + k + 32));
+    s2 += load_ro(a + k + 64) * static_cast<double>(load_ro(b + k + 64));
+    s3 += load_ro(a + k + 96) * static_cast<double>(load_ro(b + k + 96));
   }
-  for (; k < n; k += 32) s0 += a[k] * static_cast<double>(b[k]);
+  for (; k < n; k += 32) s0 += load_ro(a + k) * static_cast<double>(load_ro(b + k));
   double s = (s0 + s1) + (s2 + s3);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -797,17 +794,16 @@ __device__ __forceinline__ double gemv_row(const double *__restrict__ a,
 
 // x = Ainv b, one warp per row, FP64 accumulation
 template <typename T>
-__global__ void k_coarse_gemv(int64_t n, const double *__restrict__ A,
-                              const T *__restrict__ b, T *__restrict__ x) {
+__global__ void k_coarse_gemv(int64_t n, const double *A, const T *b, T *__restrict__ x) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   pdl_wait();
-  pdl_launch_dependents();
   for (int64_t row = warp; row < n; row += nwarps) {
     const double s = gemv_row(A + row * n, b, n, lane);
     if (lane == 0) x[row] = static_cast<T>(s);
   }
+  pdl_launch_dependents();
 }
 
 // Chebyshev start: r = D^-1 (b or the residual already in r), d = r/theta,

@@ -95,8 +95,7 @@ __global__ void __launch_bounds__(kRedThreads)
 // p = z (first) or p = z + (rho / rho_old) p, per column; a frozen column
 // keeps its p
 template <typename T>
-__global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
-                       const double *__restrict__ scal, bool first) {
+__global__ void k_cg_p(int64_t n, const T *z, T *p, const double *scal, bool first) {
   using VT = Vec16<T>;
   using V = typename VT::V;
   pdl_wait();
@@ -114,7 +113,7 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
     const V *zv = reinterpret_cast<const V *>(z);
     V *pv = reinterpret_cast<V *>(p);
     for (int64_t i = t0; i < nv; i += st) {
-      const V zz = zv[i];
+      const V zz = load_ro(zv + i);
       V pp = first ? zz : pv[i];
       if (!first) {
 #pragma unroll
@@ -124,7 +123,10 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
     }
     tail = nv * VT::W;
   }
-  for (int64_t i = tail + t0; i < n; i += st) p[i] = first ? z[i] : z[i] + beta * p[i];
+  for (int64_t i = tail + t0; i < n; i += st) {
+    const T zi = load_ro(z + i);
+    p[i] = first ? zi : zi + beta * p[i];
+  }
   pdl_launch_dependents();
 }
 
@@ -133,8 +135,7 @@ __global__ void k_cg_p(int64_t n, const T *__restrict__ z, T *__restrict__ p,
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads)
     k_cg_update(int64_t n, T *__restrict__ x, T *__restrict__ r,
-                const T *__restrict__ p, const T *__restrict__ q,
-                const double *__restrict__ scal, double *part,
+                const T *p, const T *q, const double *scal, double *part,
                 unsigned int *ticket, double *rr) {
   using VT = Vec16<T>;
   using V = typename VT::V;
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kRedThreads)
       V rr_ = rv[i];
       if (!frozen) {
         V xx = xv[i];
-        const V pp = pv[i], qq = qv[i];
+        const V pp = load_ro(pv + i), qq = load_ro(qv + i);
 #pragma unroll
         for (int k = 0; k < VT::W; ++k) {
           VT::set(xx, k, VT::get(xx, k) + alpha * VT::get(pp, k));
@@ -179,8 +180,8 @@ __global__ void __launch_bounds__(kRedThreads)
   for (int64_t i = tail + t0; i < n; i += st) {
     T ri = r[i];
     if (!frozen) {
-      x[i] += alpha * p[i];
-      ri -= alpha * q[i];
+      x[i] += alpha * load_ro(p + i);
+      ri -= alpha * load_ro(q + i);
       r[i] = ri;
     }
     s += static_cast<double>(ri) * static_cast<double>(ri);
