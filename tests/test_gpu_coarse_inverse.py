@@ -65,3 +65,17 @@ def test_inverse_is_as_accurate_as_lapack(T):
             got, ref = energy_errors(t, K, free, np.linalg.inv(K), 12)
             ratio.append(got / ref)
     assert np.exp(np.mean(np.log(ratio))) < np.sqrt(2.0)
+
+
+@pytest.mark.parametrize("nel", [(150, 1, 1), (300, 1, 1)])
+def test_inverse_of_a_slender_beam(T, nel):
+    """A backward stable factorisation leaves an error of some u cond(K) at
+    most in the energy norm, also where cond(K) is 1e11; CG with such an inverse
+    converges at once."""
+    for kind in ("uniform", "smooth", "rough"):
+        t, K, free = operator(T, nel, kind)
+        w = np.linalg.eigvalsh(K)
+        got, _ = energy_errors(t, K, free, np.linalg.inv(K), 4)
+        assert got <= 1.1e-16 * w[-1] / w[0]
+        t.FESolve(T.default_opts(rtol=1e-8, precision=T.PREC_FP64))
+        assert t.last_solve["status"] == 0 and t.last_solve["iterations"] <= 3

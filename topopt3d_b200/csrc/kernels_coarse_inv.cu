@@ -108,9 +108,13 @@ __device__ __forceinline__ void d_to_a(double d0, double d1, int lane, double &a
 // -M^-1 of the symmetric T x T tile whose 8-row strip w each warp holds in
 // acc (D fragments of T / 8 blocks), by sweeps of 8 x 8 pivots: the block
 // column of the pivot goes to shared memory, every warp inverts the pivot
-// block for itself (scalar Gauss-Jordan by shuffles; one barrier per pivot)
-// and updates its strip with tensor-core MMAs.  A pivot that is not
-// positive records its dof + 1 in *info (the first one wins).
+// block for itself (one barrier per pivot) and updates its strip with
+// tensor-core MMAs.  The pivot block is factorised by shuffles, M = L D L^T, L^-1
+// taking the place of L, and its inverse formed as L^-T D^-1 L^-1: by
+// Gauss-Jordan steps in place the inverse loses its symmetry to rounding, and the
+// soft modes of a slender beam with it (300 x 1 x 1 elements: relative error of
+// K^-1 r in the energy norm 0.2, now 1e-6).  A pivot that is not positive records its
+// dof + 1 in *info (the first one wins).
 // Fs: 2 x T x 12 doubles.
 template <int T>
 __device__ __forceinline__ void invert_tile(double (&acc)[T / 8][2], double *Fs, const int *dof,
@@ -123,7 +127,7 @@ __device__ __forceinline__ void invert_tile(double (&acc)[T / 8][2], double *Fs,
         make_double2(acc[kb][0], acc[kb][1]);
     __syncthreads();
     const double2 m = *reinterpret_cast<const double2 *>(F + (8 * kb + g) * 12 + 2 * q);
-    double m0 = m.x, m1 = m.y;
+    double m0 = m.x, m1 = m.y, ipa = 0.0, ipb = 0.0;   // 1 / D of rows q and 4 + q
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const double ms = (k & 1) ? m1 : m0;
@@ -134,12 +138,28 @@ __device__ __forceinline__ void invert_tile(double (&acc)[T / 8][2], double *Fs,
       const bool ok = p > 0.0 && p < INFINITY;
       if (!ok && threadIdx.x == 0) atomicCAS(info, 0, dof[8 * kb + k] + 1);
       const double ip = ok ? 1.0 / p : 0.0;
-      const double r0 = rk0 * ip, r1 = rk1 * ip;
-      m0 = g == k ? r0 : fma(-ck, r0, m0);
-      m1 = g == k ? r1 : fma(-ck, r1, m1);
-      if (2 * q == k) m0 = g == k ? ip : -ck * ip;
-      if (2 * q + 1 == k) m1 = g == k ? ip : -ck * ip;
+      if (q == (k & 3)) (k < 4 ? ipa : ipb) = ip;
+      if (g > k) {   // rows below: of M right of the pivot, of L^-1 left of it
+        const double l = ck * ip;
+        m0 = 2 * q == k ? -l : fma(-l, rk0, m0);
+        m1 = 2 * q + 1 == k ? -l : fma(-l, rk1, m1);
+      }
     }
+    // L^-1[q][g], L^-1[4 + q][g]: B fragments of L^-1 and A fragments of L^-T
+    double l0, l1;
+    {
+      const int s = 4 * q + (g >> 1);
+      const double x0 = __shfl_sync(0xffffffffu, m0, s), x1 = __shfl_sync(0xffffffffu, m1, s);
+      const double y0 = __shfl_sync(0xffffffffu, m0, s + 16);
+      const double y1 = __shfl_sync(0xffffffffu, m1, s + 16);
+      l0 = g < q ? ((g & 1) ? x1 : x0) : (g == q ? 1.0 : 0.0);
+      l1 = g < 4 + q ? ((g & 1) ? y1 : y0) : (g == 4 + q ? 1.0 : 0.0);
+    }
+    double pd[2] = {0.0, 0.0};
+    dmma(pd, l0 * ipa, l0);
+    dmma(pd, l1 * ipb, l1);
+    m0 = pd[0];
+    m1 = pd[1];
     // P8 = (m0, m1); it is symmetric, so its A fragments are its B
     // fragments too
     double p0, p1;
