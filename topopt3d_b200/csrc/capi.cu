@@ -235,15 +235,16 @@ int alloc_solver(Ctx &c) {
   }
   if (c.L > 2) A(c.gd_tmp, tpo::galerkin_dims_scratch(c.lev[1]));
   const int64_t nc = 3 * c.lev[c.L - 1].nn;
-  if (!c.inv.dev) {
+  if (!c.inv.dev) {   // inversion workspace and plan
     tpo::coarse_inverse_plan(c.lev[c.L - 1].dims, c.inv);
-    A(c.inv.dev, c.inv.host.size());
-    CK(cudaMemcpyAsync(c.inv.dev, c.inv.host.data(), sizeof(int) * c.inv.host.size(),
-                       cudaMemcpyHostToDevice, c.stream));
-    CK(cudaStreamSynchronize(c.stream));
-    c.inv.host = std::vector<int>();
+    const size_t work = tpo::coarse_inverse_work(c.inv);
+    A(c.Adense, work + (c.inv.ints + 1) / 2);
+    c.inv.dev = reinterpret_cast<int *>(c.Adense + work);
+    if (cudaError_t e = tpo::coarse_inverse_upload(c.inv, c.stream); e != cudaSuccess) {
+      c.inv.dev = nullptr;
+      CK(e);
+    }
   }
-  A(c.Adense, tpo::coarse_inverse_work(c.inv));   // inversion workspace
   A(c.Ainv, (size_t)(nc * nc));
   A(c.w64, 3 * c.nn);
 #undef A
@@ -263,7 +264,7 @@ void free_all(Ctx &c) {
   dfree(c.gk_G); c.gk_cap = 0; dfree(c.gd_tmp);
   dfree(c.l1_B); dfree(c.l1_rows); dfree(c.l1_C); c.l1_cap = 0; dfree(c.l1_cval);
   dfree(c.l1_cflag); dfree(c.l1_count); dfree(c.l1_fault); c.l1_bimg_ready = false;
-  dfree(c.Ainv); dfree(c.Adense); dfree(c.inv.dev); dfree(c.dev_info);
+  dfree(c.Ainv); dfree(c.Adense); c.inv.dev = nullptr; dfree(c.dev_info);
   dfree(c.finv); dfree(c.taps_d);
   dfree(c.w64);
   dfree(c.Es64); dfree(c.dEsdz64); dfree(c.bk_buf); c.bk_n = 0; dfree(c.fq_buf); c.fq_n = 0; dfree(c.mma_buf); c.mma_n = 0;

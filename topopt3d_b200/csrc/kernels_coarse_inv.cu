@@ -42,8 +42,10 @@
 // x 24 mesh 0.67 -> 0.60 ms, of 12 x 6 x 6 0.247 -> 0.227.
 #include <algorithm>
 #include <cmath>
-#include <cstring>
+#include <new>
 #include <vector>
+
+#include <sys/mman.h>
 
 #include "pdl.cuh"
 #include "tpo_internal.h"
@@ -417,8 +419,25 @@ void run_steps(const CoarseInvPlan &pl, double *work, int *info, cudaStream_t s)
 
 }  // namespace
 
+template <typename E>
+E *CoarseInvPlan::HugePages<E>::allocate(size_t n) {
+  constexpr size_t kPage = 2u << 20;
+  const size_t bytes = n * sizeof(E);
+  void *p = nullptr;
+  if (bytes < kPage) {
+    p = std::malloc(bytes);
+  } else if (posix_memalign(&p, kPage, (bytes + kPage - 1) / kPage * kPage) == 0) {
+    madvise(p, (bytes + kPage - 1) / kPage * kPage, MADV_HUGEPAGE);   // a hint
+  } else {
+    p = nullptr;
+  }
+  if (!p) throw std::bad_alloc();
+  return static_cast<E *>(p);
+}
+
 // The blocks, the elimination order and the task lists of a level of d[0] x
-// d[1] x d[2] nodes (host arrays in pl.host; the caller uploads them).
+// d[1] x d[2] nodes (on the host; coarse_inverse_upload takes them to the
+// device).
 void coarse_inverse_plan(const int d[3], CoarseInvPlan &pl) {
   const int D = (d[0] >= d[1] && d[0] >= d[2]) ? 0 : (d[1] >= d[2] ? 1 : 2);
   const int planes = d[D];
@@ -451,19 +470,26 @@ void coarse_inverse_plan(const int d[3], CoarseInvPlan &pl) {
           dofs[p] = 3 * n + r;
         }
       }
-  // coupled block pairs
+  // coupled block pairs (a node's three unknowns are in one or two blocks)
   std::vector<uint8_t> nz((size_t)nb * nb, 0);
+  const int nn = d[0] * d[1] * d[2];
+  std::vector<int> lo(nn), hi(nn);
+  for (int n = 0; n < nn; ++n) {
+    lo[n] = pos[3 * n] / T;
+    hi[n] = pos[3 * n + 2] / T;
+  }
   for (int k = 0; k < d[2]; ++k)
     for (int j = 0; j < d[1]; ++j)
-      for (int i = 0; i < d[0]; ++i)
-        for (int b = 0; b < 27; ++b) {
-          const int mi = i + b % 3 - 1, mj = j + (b / 3) % 3 - 1, mk = k + b / 9 - 1;
-          if (mi < 0 || mj < 0 || mk < 0 || mi >= d[0] || mj >= d[1] || mk >= d[2]) continue;
-          const int n = (k * d[1] + j) * d[0] + i, q = (mk * d[1] + mj) * d[0] + mi;
-          for (int r = 0; r < 3; ++r)
-            for (int s = 0; s < 3; ++s)
-              nz[(size_t)(pos[3 * n + r] / T) * nb + pos[3 * q + s] / T] = 1;
-        }
+      for (int i = 0; i < d[0]; ++i) {
+        const int n = (k * d[1] + j) * d[0] + i;
+        for (int mk = std::max(k - 1, 0); mk <= std::min(k + 1, d[2] - 1); ++mk)
+          for (int mj = std::max(j - 1, 0); mj <= std::min(j + 1, d[1] - 1); ++mj)
+            for (int mi = std::max(i - 1, 0); mi <= std::min(i + 1, d[0] - 1); ++mi) {
+              const int q = (mk * d[1] + mj) * d[0] + mi;
+              for (int a : {lo[n], hi[n]})
+                for (int b : {lo[q], hi[q]}) nz[(size_t)a * nb + b] = 1;
+            }
+      }
   // rounds of alternate plane groups; block b of every group of a round is
   // one step as long as the groups are uncoupled
   std::vector<std::vector<int>> steps;
@@ -499,8 +525,17 @@ void coarse_inverse_plan(const int d[3], CoarseInvPlan &pl) {
     }
     chain.swap(rest);
   }
-  // task lists
-  std::vector<int> fg, up, pairs;
+  // task lists.  A step's F and G tiles are numbered row block by row block
+  // within a pivot; row[I] lists those of row block I as (pivot, number), in the
+  // order of the pivots, and a tile (I, J) is updated by the pivots that both
+  // rows have (a merge: levels of 4,000 nodes have some 200,000 such pairs)
+  using Pair = CoarseInvPlan::Pair;
+  CoarseInvPlan::List<CoarseInvPlan::Task> fg, up;
+  CoarseInvPlan::List<Pair> pairs;
+  std::vector<std::vector<Pair>> row(nb);
+  std::vector<int> rows;   // those that a pivot of the step couples
+  std::vector<int> slot(nb);
+  std::vector<uint8_t> is_piv(nb);
   st = nz;
   pl.max_pivots = 1;
   pl.max_fg = 1;
@@ -509,61 +544,93 @@ void coarse_inverse_plan(const int d[3], CoarseInvPlan &pl) {
     const std::vector<int> &piv = steps[q];
     pl.max_pivots = std::max(pl.max_pivots, (int)piv.size());
     CoarseInvPlan::Step S{};
-    S.fg = (int)(fg.size() / 4);
-    S.up = (int)(up.size() / 4);
-    std::vector<uint8_t> is_piv(nb, 0);
+    S.fg = (int)fg.size();
+    S.up = (int)up.size();
+    std::fill(is_piv.begin(), is_piv.end(), 0);
     for (int k : piv) is_piv[k] = 1;
-    // index of (I, pivot) among this step's F and G tiles, per row block
-    std::vector<std::vector<std::pair<int, int>>> of(nb);
+    for (auto &r : row) r.clear();
     int nfg = 0;
     for (size_t p = 0; p < piv.size(); ++p)
       for (int I = 0; I < nb; ++I)
         if (I != piv[p] && coupled(I, piv[p])) {
-          of[I].push_back({(int)p, nfg++});
-          fg.insert(fg.end(), {I, piv[p], (int)p, 0});
+          row[I].push_back({(int)p, nfg++});
+          fg.push_back({{I, piv[p], (int)p, 0}});
         }
     S.nfg = nfg;
     pl.max_fg = std::max(pl.max_fg, nfg);
-    std::vector<int> slot(nb, -1);
+    rows.clear();
+    for (int I = 0; I < nb; ++I)
+      if (!is_piv[I] && !row[I].empty()) rows.push_back(I);
+    std::fill(slot.begin(), slot.end(), -1);
     if (q + 1 < steps.size())
       for (size_t p = 0; p < steps[q + 1].size(); ++p) slot[steps[q + 1][p]] = (int)p;
     auto task = [&](int I, int J) {
       const int next = I == J ? slot[I] : -1;
-      const int first = (int)(pairs.size() / 2);
-      int cnt = 0;
-      if (!is_piv[I] && !is_piv[J])
-        for (auto &a : of[I])
-          for (auto &b : of[J])
-            if (a.first == b.first) {
-              pairs.insert(pairs.end(), {a.second, b.second});
-              ++cnt;
-            }
-      if (cnt || next >= 0) up.insert(up.end(), {I | (J << 16), first, cnt, next});
+      const int first = (int)pairs.size();
+      if (!is_piv[I] && !is_piv[J]) {
+        const Pair *x = row[I].data(), *xe = x + row[I].size();
+        const Pair *y = row[J].data(), *ye = y + row[J].size();
+        while (x != xe && y != ye) {
+          if (x->a == y->a) pairs.push_back({x->b, y->b});
+          const bool nx = x->a <= y->a, ny = y->a <= x->a;
+          x += nx;
+          y += ny;
+        }
+      }
+      const int cnt = (int)pairs.size() - first;
+      if (cnt || next >= 0) up.push_back({{I | (J << 16), first, cnt, next}});
     };
     for (int I = 0; I < nb; ++I)   // the next step's pivots first
       if (slot[I] >= 0) task(I, I);
-    for (int I = 0; I < nb; ++I)
-      for (int J = 0; J <= I; ++J)
+    for (int I : rows)
+      for (int J : rows) {
+        if (J > I) break;
         if (!(I == J && slot[I] >= 0)) task(I, J);
-    S.nup = (int)(up.size() / 4) - S.up;
+      }
+    S.nup = (int)up.size() - S.up;
     pl.steps.push_back(S);
     for (int k : piv) eliminate(k);
   }
   pl.first_pivots = (int)steps[0].size();
   // one device array; the task lists (int4, int2) first, for their alignment
-  pl.host.clear();
-  auto put = [&](const std::vector<int> &v) {
-    const size_t o = pl.host.size();
-    pl.host.insert(pl.host.end(), v.begin(), v.end());
-    while (pl.host.size() % 4) pl.host.push_back(0);
+  pl.ints = 0;
+  auto put = [&](size_t bytes) {
+    const size_t o = pl.ints;
+    pl.ints += (bytes + 15) / 16 * 4;
     return o;
   };
-  pl.off_fg = put(fg);
-  pl.off_up = put(up);
-  pl.off_pairs = put(pairs);
-  pl.off_piv = put(steps[0]);
-  pl.off_dofs = put(dofs);
-  pl.off_pos = put(pos);
+  pl.piv = steps[0];
+  pl.fg.swap(fg);
+  pl.up.swap(up);
+  pl.pairs.swap(pairs);
+  pl.dofs.swap(dofs);
+  pl.pos.swap(pos);
+  pl.off_fg = put(sizeof(pl.fg[0]) * pl.fg.size());
+  pl.off_up = put(sizeof(pl.up[0]) * pl.up.size());
+  pl.off_pairs = put(sizeof(pl.pairs[0]) * pl.pairs.size());
+  pl.off_piv = put(sizeof(int) * pl.piv.size());
+  pl.off_dofs = put(sizeof(int) * pl.dofs.size());
+  pl.off_pos = put(sizeof(int) * pl.pos.size());
+}
+
+cudaError_t coarse_inverse_upload(CoarseInvPlan &pl, cudaStream_t s) {
+  cudaError_t err = cudaSuccess;
+  auto copy = [&](size_t off, const auto &v) {
+    if (!v.empty() && err == cudaSuccess)
+      err = cudaMemcpyAsync(pl.dev + off, v.data(), sizeof(v[0]) * v.size(),
+                            cudaMemcpyHostToDevice, s);
+  };
+  copy(pl.off_fg, pl.fg);
+  copy(pl.off_up, pl.up);
+  copy(pl.off_pairs, pl.pairs);
+  copy(pl.off_piv, pl.piv);
+  copy(pl.off_dofs, pl.dofs);
+  copy(pl.off_pos, pl.pos);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+  pl.fg = pl.up = {};
+  pl.pairs = {};
+  pl.piv = pl.dofs = pl.pos = {};
+  return err;
 }
 
 size_t coarse_inverse_work(const CoarseInvPlan &pl) {

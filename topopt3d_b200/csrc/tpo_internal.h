@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -95,18 +96,42 @@ struct Level {
 
 // The coarsest inverse's elimination plan (kernels_coarse_inv.cu): tile size,
 // blocks, unknowns, the steps' ranges in the task lists, and the lists
-// (offsets into one int array, host until uploaded, then dev)
+// (offsets into one int array `dev`, which is filled by coarse_inverse_upload)
 struct CoarseInvPlan {
   struct Step {
     int fg, nfg, up, nup;
   };
+  struct Task {
+    int v[4];
+  };
+  struct Pair {
+    int a, b;
+  };
+  // the lists on the host until they are uploaded (one level of 4,000 nodes
+  // has 1.9 M ints of them): on huge pages, since a fault for each 4 KB took
+  // most of the time that building them does
+  template <typename E>
+  struct HugePages {
+    using value_type = E;
+    HugePages() = default;
+    template <typename F>
+    HugePages(const HugePages<F> &) {}
+    E *allocate(size_t n);
+    void deallocate(E *p, size_t) { std::free(p); }
+    bool operator==(const HugePages &) const { return true; }
+    bool operator!=(const HugePages &) const { return false; }
+  };
+  template <typename E>
+  using List = std::vector<E, HugePages<E>>;
   int T = 0, nb = 0;
   int64_t n = 0;
   int first_pivots = 0, max_pivots = 0, max_fg = 0;
   std::vector<Step> steps;
-  std::vector<int> host;
-  size_t off_fg = 0, off_up = 0, off_pairs = 0, off_piv = 0, off_dofs = 0, off_pos = 0;
-  int *dev = nullptr;
+  List<Task> fg, up;
+  List<Pair> pairs;
+  std::vector<int> piv, dofs, pos;
+  size_t ints = 0, off_fg = 0, off_up = 0, off_pairs = 0, off_piv = 0, off_dofs = 0, off_pos = 0;
+  int *dev = nullptr;   // behind the inversion workspace
 };
 
 // side streams of the set-up (per-level power iterations)
@@ -441,6 +466,8 @@ void launch_coarse_slabs(const Level &v, int ctas, const double *S, double *A64,
 // (kernels_coarse_inv.cu); work holds coarse_inverse_work(plan) doubles;
 // *info becomes the index + 1 of the first dof whose pivot is not positive
 void coarse_inverse_plan(const int dims[3], CoarseInvPlan &plan);
+// the lists to plan.dev (plan.ints ints), and off the host
+cudaError_t coarse_inverse_upload(CoarseInvPlan &plan, cudaStream_t s);
 size_t coarse_inverse_work(const CoarseInvPlan &plan);
 void launch_coarse_inverse(const Level &v, const double *S, const CoarseInvPlan &plan,
                            double *Ainv, double *work, int *info, cudaStream_t s);
