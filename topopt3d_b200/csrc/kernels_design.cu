@@ -90,14 +90,20 @@ __global__ void k_filter_adj(int nx, int ny, int nz,
 // w[|j|]; a thread forms four outputs along y, whose columns share their
 // values: 4 + 2n reads for 4 (2n + 1) products.  Values outside the mesh are
 // zeros, taps outside the cone are never formed.  The forward form scales the
-// sum by finv, the transposed one the values.  (One thread per output with
-// its taps' offsets and weights read from memory and each one checked against
-// the mesh took 80 us a pass at 128x64x64 with 93 taps, 55 and 72 us at
-// 192x96x96 with 19; this form takes 27, 28 and 26 us, where the copy of the
-// bytes takes 1.3 and 4.4 us: it is bound by its shared-memory reads and the
-// one wait for the tile.)
+// sum by finv, the transposed one the values.
+//
+// One thread per output with its taps' offsets and weights read from memory and
+// each one checked against the mesh takes, forward and transposed, 68 and 93 us
+// at 128x64x64 with 93 taps, 53 and 70 us at 192x96x96 with 19, 16.6 and 22.7 us
+// at 64x32x32 with 93 and 6.4 and 8.4 us there with 19; this form takes 15.6,
+// 18.6, 10.4 and 6.6 and 8.3 us.  (The copy of the bytes takes 1.3 and 4.4 us at
+// the first two: it is bound by its shared-memory reads and the one wait for
+// the tile.)  Sixteen warps a CTA, one z plane of the tile to each four: with
+// four warps for all of them the load of the tile is a chain of 29 to 63 trips a
+// thread, the same four cases took 31 and 23, 23 and 21, 28 and 21, and 15.6 and
+// 12.5 us, and small meshes were slower than with a thread per output.
 constexpr int kFtMax = 3;
-constexpr int kFtX = 32, kFtY = 16, kFtZ = 4, kFtThreads = 128;
+constexpr int kFtX = 32, kFtY = 16, kFtZ = 4, kFtThreads = 128 * kFtZ;
 struct FilterColumns {
   int n;
   struct {
@@ -132,6 +138,7 @@ __global__ void __launch_bounds__(kFtThreads)
   for (int t = threadIdx.x; t < (int)(sizeof(FilterColumns) / 4); t += kFtThreads)
     reinterpret_cast<int *>(&sc)[t] = reinterpret_cast<const int *>(&cols)[t];
   const int x0 = blockIdx.x * kFtX - H, y0 = blockIdx.y * kFtY - H, z0 = blockIdx.z * kFtZ - H;
+#pragma unroll 4
   for (int t = threadIdx.x; t < SX * SY * SZ; t += kFtThreads) {
     const int x = x0 + t % SX, y = y0 + (t / SX) % SY, z = z0 + t / (SX * SY);
     double v = 0.0;
@@ -142,31 +149,31 @@ __global__ void __launch_bounds__(kFtThreads)
     }
     tile[t] = v;
   }
-  __syncthreads();
-  const int tx = threadIdx.x & 31, ty = 4 * (threadIdx.x >> 5);
-  const int x = x0 + H + tx, y = y0 + H + ty;
-#pragma unroll 1
-  for (int k = 0; k < kFtZ; ++k) {
-    const int z = z0 + H + k;
-    if (z >= nz) break;   // uniform over the CTA
-    const double *v = tile + ((k + H) * SY + ty + H) * SX + tx + H;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-    for (int c = 0; c < sc.n; ++c) {
-      const double *w = sc.c[c].w, *p = v + sc.c[c].at;
-      const int ext = sc.c[c].ext;   // uniform
-      if (ext == 0) filter_column<0>(p, SX, w, acc);
-      else if (ext == 1) filter_column<1>(p, SX, w, acc);
-      else if (H >= 2 && ext == 2) filter_column<H >= 2 ? 2 : 1>(p, SX, w, acc);
-      else if (H >= 3) filter_column<H >= 3 ? 3 : 1>(p, SX, w, acc);
-    }
+  const int tx = threadIdx.x & 31, ty = 4 * ((threadIdx.x >> 5) & 3), k = threadIdx.x >> 7;
+  const int x = x0 + H + tx, y = y0 + H + ty, z = z0 + H + k;
+  const int64_t e0 = ((int64_t)z * ny + y) * nx + x;
+  double f[4];
+  if (!ADJ) {
 #pragma unroll
     for (int o = 0; o < 4; ++o)
-      if (x < nx && y + o < ny) {
-        const int64_t e = ((int64_t)z * ny + y + o) * nx + x;
-        out[e] = ADJ ? acc[o] : acc[o] * finv[e];
-      }
+      f[o] = x < nx && y + o < ny && z < nz ? finv[e0 + (int64_t)o * nx] : 0.0;
   }
+  __syncthreads();
+  if (z >= nz) return;   // uniform over a warp
+  const double *v = tile + ((k + H) * SY + ty + H) * SX + tx + H;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int c = 0; c < sc.n; ++c) {
+    const double *w = sc.c[c].w, *p = v + sc.c[c].at;
+    const int ext = sc.c[c].ext;   // uniform
+    if (ext == 0) filter_column<0>(p, SX, w, acc);
+    else if (ext == 1) filter_column<1>(p, SX, w, acc);
+    else if (H >= 2 && ext == 2) filter_column<H >= 2 ? 2 : 1>(p, SX, w, acc);
+    else if (H >= 3) filter_column<H >= 3 ? 3 : 1>(p, SX, w, acc);
+  }
+#pragma unroll
+  for (int o = 0; o < 4; ++o)
+    if (x < nx && y + o < ny) out[e0 + (int64_t)o * nx] = ADJ ? acc[o] : acc[o] * f[o];
 }
 
 // PETSc VecPow special cases (used by MatIntFnc)
@@ -716,22 +723,21 @@ static int filter_columns(const FilterTaps &taps, FilterColumns &f) {
     for (int d = 0; d < 3; ++d) H = std::max(H, std::abs((int)taps.off[t][d]));
   if (H > kFtMax) return H;
   H = std::max(H, 1);
-  const int SX = kFtX + 2 * H, SY = kFtY + 2 * H;
+  const int SX = kFtX + 2 * H, SY = kFtY + 2 * H, S = 2 * H + 1;
+  for (int q = 0; q < S * S; ++q) f.c[q].ext = -1;
+  for (int t = 0; t < taps.n; ++t) {
+    const int i = taps.off[t][0], j = taps.off[t][1], k = taps.off[t][2];
+    if (j < 0) continue;
+    auto &c = f.c[(k + H) * S + i + H];
+    c.ext = std::max(c.ext, (short)j);
+    c.w[j] = taps.w[t];
+  }
   f.n = 0;
-  for (int k = -H; k <= H; ++k)
-    for (int i = -H; i <= H; ++i) {
-      auto &c = f.c[f.n];
-      int ext = -1;
-      for (int t = 0; t < taps.n; ++t)
-        if (taps.off[t][2] == k && taps.off[t][0] == i && taps.off[t][1] >= 0) {
-          ext = std::max(ext, (int)taps.off[t][1]);
-          c.w[taps.off[t][1]] = taps.w[t];
-        }
-      if (ext < 0) continue;
-      c.ext = (short)ext;
-      c.at = (short)(k * SX * SY + i);
-      ++f.n;
-    }
+  for (int q = 0; q < S * S; ++q) {
+    if (f.c[q].ext < 0) continue;
+    f.c[f.n] = f.c[q];
+    f.c[f.n++].at = (short)((q / S - H) * SX * SY + q % S - H);
+  }
   return H;
 }
 
@@ -751,20 +757,23 @@ static void filter_tile(const Ctx &c, const FilterColumns &f, const double *in, 
                                                     uniform, out);
 }
 
-// tiles up to kFtMax elements of halo (radii below 4 elements) and meshes
-// that fit the grid, else one thread per output
+// tiles up to kFtMax elements of halo (radii up to 4 elements) and meshes
+// that fit the grid, else one thread per output; that also for a template of
+// one tap (radii up to 1), which shares nothing: 6.4 us at 128x64x64 for the
+// tiles' 8.3
 template <bool ADJ>
 static void filter_any(const Ctx &c, const double *in, double uniform, double *out,
                        cudaStream_t s) {
   FilterColumns f{};
-  const int H = filter_columns(c.taps, f);
-  const bool fits = (c.nel[1] + kFtY - 1) / kFtY <= 65535 && (c.nel[2] + kFtZ - 1) / kFtZ <= 65535;
+  const bool fits = c.taps.n > 1 && (c.nel[1] + kFtY - 1) / kFtY <= 65535 &&
+                    (c.nel[2] + kFtZ - 1) / kFtZ <= 65535;
+  const int H = fits ? filter_columns(c.taps, f) : kFtMax + 1;
   count_launch();
-  if (H <= 1 && fits)
+  if (H <= 1)
     filter_tile<1, ADJ>(c, f, in, uniform, out, s);
-  else if (H == 2 && fits)
+  else if (H == 2)
     filter_tile<2, ADJ>(c, f, in, uniform, out, s);
-  else if (H == 3 && fits)
+  else if (H == 3)
     filter_tile<3, ADJ>(c, f, in, uniform, out, s);
   else if (ADJ)
     k_filter_adj<<<grid_for(c.ne, 256), 256, 0, s>>>(c.nel[0], c.nel[1], c.nel[2], c.taps_d,
