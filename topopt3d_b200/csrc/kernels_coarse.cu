@@ -472,22 +472,26 @@ __global__ void __launch_bounds__(Shape<T, NB, SPLIT>::kThreads, 1)
   if (failed) *(volatile double *)P.fault = 1.0;
 }
 
-// shared memory per CTA, once per device; 0 when the attribute cannot be set
+// shared memory per CTA, found and opted in to once per device
 template <typename T, int NB, int SPLIT>
-size_t smem_limit(int dev) {
+cudaError_t smem_limit(int dev, size_t *limit) {
   static size_t cached[64] = {0};
   size_t &c = cached[dev & 63];
   if (!c) {
     int opt = 0;
     cudaFuncAttributes fa{};
-    cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncGetAttributes(&fa, (const void *)k_coarse_cycle<T, NB, SPLIT>);
+    cudaError_t err = cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (err == cudaSuccess)
+      err = cudaFuncGetAttributes(&fa, (const void *)k_coarse_cycle<T, NB, SPLIT>);
+    if (err != cudaSuccess) return err;
     const size_t lim = ((size_t)opt - fa.sharedSizeBytes) / 128 * 128;
-    cudaFuncSetAttribute(k_coarse_cycle<T, NB, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)lim);
+    err = cudaFuncSetAttribute(k_coarse_cycle<T, NB, SPLIT>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim);
+    if (err != cudaSuccess) return err;
     c = lim;
   }
-  return c;
+  *limit = c;
+  return cudaSuccess;
 }
 
 template <typename T, int NB, int SPLIT>
@@ -495,7 +499,8 @@ cudaError_t launch_split(CoarseCycle<T> &P, cudaStream_t s) {
   using Sh = Shape<T, NB, SPLIT>;
   int dev = 0;
   cudaGetDevice(&dev);
-  const size_t lim = smem_limit<T, NB, SPLIT>(dev);
+  size_t lim = 0;
+  if (cudaError_t err = smem_limit<T, NB, SPLIT>(dev, &lim); err != cudaSuccess) return err;
   // partial sums of up to kPartCap bytes, then the resident rows
   int npc = 32;
   for (int l = 0; l < P.nlev; ++l) npc = npc > P.lev[l].npc ? npc : P.lev[l].npc;
@@ -506,6 +511,7 @@ cudaError_t launch_split(CoarseCycle<T> &P, cudaStream_t s) {
   const size_t dense = sizeof(double) * Sh::kWarps * NB;
   if (used < dense) used = dense;
   used = (used + 127) / 128 * 128;
+  if (used > lim) return cudaErrorInvalidConfiguration;
   // the small levels whole first (their phases are pure latency), then what
   // fits of the top level
   for (int l = P.nlev - 1; l >= 0; --l) {
