@@ -839,10 +839,12 @@ bool launch_oc_bisect(const Ctx &c, int64_t n, double *x, const double *xold,
   cudaGetDevice(&dev);
   dev &= 63;
   if (!ctas[dev]) {
-    int per_sm = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oc_bisect<2>, kOcThreads, 0);
+    int a = 0, b = 0, d = 0, sms = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_oc_bisect<0>, kOcThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_oc_bisect<1>, kOcThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_oc_bisect<2>, kOcThreads, 0);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ctas[dev] = per_sm > 0 ? std::min(sms, kRedBlocks) : -1;
+    ctas[dev] = a > 0 && b > 0 && d > 0 ? std::min(sms, kRedBlocks) : -1;
   }
   if (ctas[dev] < 0) return false;
   count_launch();
