@@ -780,12 +780,12 @@ __device__ __forceinline__ double gemv_row(const double *a, const T *b, int64_t 
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
   int64_t k = lane;
   for (; k + 96 < n; k += 128) {
-    s0 += load_ro(a + k) * static_cast<double>(load_ro(b + k));
-    s1 += load_ro(a + k + 32) * static_cast<double>(load_ro(b + k + 32));
-    s2 += load_ro(a + k + 64) * static_cast<double>(load_ro(b + k + 64));
-    s3 += load_ro(a + k + 96) * static_cast<double>(load_ro(b + k + 96));
+    s0 += a[k] * static_cast<double>(b[k]);
+    s1 += a[k + 32] * static_cast<double>(b[k + 32]);
+    s2 += a[k + 64] * static_cast<double>(b[k + 64]);
+    s3 += a[k + 96] * static_cast<double>(b[k + 96]);
   }
-  for (; k < n; k += 32) s0 += load_ro(a + k) * static_cast<double>(load_ro(b + k));
+  for (; k < n; k += 32) s0 += a[k] * static_cast<double>(b[k]);
   double s = (s0 + s1) + (s2 + s3);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
