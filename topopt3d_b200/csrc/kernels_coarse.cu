@@ -34,12 +34,13 @@
 // barrier; the restriction also writes the child's first direction.
 //
 // Measured (us a cycle in a solve's launch list; before: a warp per node, 592
-// CTAs, every phase from L2; and now): 192x96x96 FP32 91 -> 65, FP64 116 ->
-// 85; 91x47x53 FP32 84 -> 57; 48x24x24 FP64 36 -> 26; 128x64x64, 8 FP32
-// columns 128 -> 74; 75x41x34 FP64, 4 columns 139 -> 85, 1 column 77 -> 50;
-// 96x48x48 FP64, 8 columns 341 -> 310, 4 columns 215 -> 167.  What is left at
-// 192x96x96 (121 k cycles): 12 barriers of 2.7 k, the first phase's 30 MB of
-// stencil from DRAM 17 k, the inverse (29 MB) 14 k, the other phases 2 - 9 k.
+// CTAs, every phase from L2, 89 and 112 by itself at 192x96x96; and now):
+// 192x96x96 FP32 91 -> 65, FP64 116 -> 85; 91x47x53 FP32 84 -> 57; 48x24x24
+// FP64 36 -> 26; 128x64x64, 8 FP32 columns 128 -> 74; 75x41x34 FP64, 4 columns
+// 139 -> 85, 1 column 77 -> 50; 96x48x48 FP64, 8 columns 341 -> 310, 4 columns
+// 215 -> 167.  What is left at 192x96x96 (121 k cycles): 12 barriers of 2.7 k,
+// the first phase's 30 MB of stencil from DRAM 17 k, the inverse (29 MB) 14 k,
+// the other phases 2 - 9 k.
 #include "coarse.h"
 #include "grid_barrier.cuh"
 #include "umma.cuh"

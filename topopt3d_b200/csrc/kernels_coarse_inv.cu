@@ -21,7 +21,7 @@
 // half the length.  A 13 x 7 x 7 level (1,911 unknowns) takes 4 rounds of 3
 // blocks of 49, 12 dependent steps, where the natural order takes 30 steps
 // of 64; tiles that no pivot of a step couples are skipped (the structure is
-// worked out once per context on the host, plan_build).
+// worked out once per context on the host, coarse_inverse_plan).
 //
 // A step is two launches over task lists: F and G of every coupled (row
 // block, pivot) pair (k_ci_fg), and the updates of the lower tiles by
@@ -36,10 +36,11 @@
 // natural order in 64-blocks took 1,480 us, 36 us a step for the update
 // with the scalar inversion of the next block (22 us of it) and 12 us for F
 // and G; this form takes 356 us (12 x (6.4 + 19.7), fill 5, first pivots 13,
-// final pass 25).  The launches of the chain are programmatic dependent ones,
-// released when a block's arithmetic is done (released at its start, the
-// waiting blocks kept those of the side streams out): FEAssemble of a 48 x 24
-// x 24 mesh 0.67 -> 0.60 ms, of 12 x 6 x 6 0.247 -> 0.227.
+// final pass 25), 3% more since the updates' sums are kept apart.  The launches
+// of the chain are programmatic dependent ones, released when a block's
+// arithmetic is done (released at its start, the waiting blocks kept those of
+// the side streams out): FEAssemble of a 48 x 24 x 24 mesh 0.67 -> 0.60 ms, of
+// 12 x 6 x 6 0.247 -> 0.227.
 #include <algorithm>
 #include <cmath>
 #include <new>
